@@ -4,6 +4,7 @@
 // slot. Slots are re-sorted by (cell, particle id) at the end of every step (inside the
 // closure kick), so per-cell work reads contiguous memory; every API that exchanges particle
 // arrays with the host uses particle-id order, as the reference does.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,6 +30,7 @@
 #include "fast_batch.cuh"
 #include "learned.cuh"
 #include "sort.cuh"
+#include "state_io.cuh"
 #include "zone.cuh"
 
 using namespace mpcd_dev;
@@ -96,6 +98,7 @@ struct mpcd_ctx {
     // positions in place and velocities out of place, so each pass flips xv and xflip together
     // (the positions stay in their buffer); a whole step leaves xflip as it found it.
     int xflip = 0;
+    int* partFill = nullptr;  // kPartBuckets: bucket fill counts of the state's id-order output (state_io.cuh)
     int* cidStd = nullptr;
     int* cidSrd = nullptr;
     uint64_t* sortKeys = nullptr;  // n: (particle id, slot) keys of the index being built
@@ -314,6 +317,9 @@ inline View32 view32(const mpcd_ctx* c, int k) {
 // positions of the current state, and the other position buffer (free as scratch)
 inline double2* cur_x(const mpcd_ctx* c) { return c->xb[c->xv ^ c->xflip]; }
 inline double2* spare_x(const mpcd_ctx* c) { return c->xb[c->xv ^ c->xflip ^ 1]; }
+// state I/O staging of an FP32 context, n double2 each: the closure's scratch, free between calls
+inline double2* f32_scratch_x(const mpcd_ctx* c) { return c->vrep; }
+inline double2* f32_scratch_v(const mpcd_ctx* c) { return reinterpret_cast<double2*>(c->cols); }
 #define WITH_VIEW(k, ...)                          \
     do {                                           \
         if (c->f32) {                              \
@@ -369,6 +375,42 @@ int check_device(mpcd_ctx* c) {
         return set_err(rc, std::string(dev_error_text(code)) + " (detail " + std::to_string(detail) + ")");
     }
     return MPCD_OK;
+}
+
+// Whether kernels may read or write a caller's device buffer in place of a staged copy: device
+// memory of `device`, aligned for double2 accesses, the whole extent inside one allocation (a
+// copy would check the extent; a kernel does not).
+bool direct_device(const void* p, size_t bytes, int device) {
+    cudaPointerAttributes a{};
+    if ((uintptr_t)p % alignof(double2) != 0 || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (a.type != cudaMemoryTypeDevice || a.device != device) return false;
+    using RangeFn = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const RangeFn range = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found{};
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return (RangeFn)fn;
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    if (!range || range(&base, &size, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+    return (CUdeviceptr)p >= base && (CUdeviceptr)p - base <= size && bytes <= size - ((CUdeviceptr)p - base);
+}
+
+// The two-pass output (state_io.cuh) pays where the output outgrows the L2 cache.
+constexpr int64_t kPartMin = 4 << 20;  // particles (128 MB of x and v)
+
+// whether two buffers of `bytes` bytes share no byte (nulls share none)
+bool disjoint(const void* a, const void* b, size_t bytes) {
+    const uintptr_t p = (uintptr_t)a, q = (uintptr_t)b;
+    return !a || !b || (p < q ? q - p : p - q) >= bytes;
 }
 
 template <typename T>
@@ -1249,6 +1291,7 @@ int mpcd_ctx_destroy(mpcd_ctx* c) {
     fast_free(c);
     if (c->profP) cudaFree(c->profP);
     if (c->profN) cudaFree(c->profN);
+    if (c->partFill) cudaFree(c->partFill);
     void* ptrs[] = {c->xb[0], c->xb[1], c->vb[0], c->vb[1], c->offb[0], c->offb[1], c->cellb[0], c->cellb[1],
                     c->v32b[0], c->v32b[1], c->pidb[0], c->pidb[1], c->cidStd, c->cidSrd, c->sortKeys, c->sortKeysSide,
                     c->idxStd.count, c->idxStd.start, c->idxStd.pos, c->idxStd.slots,
@@ -1326,6 +1369,7 @@ int mpcd_ctx_create_form(const mpcd_params_c* params, int device, int32_t form, 
     if (cudaSetDevice(device) != cudaSuccess) return fail(set_err(MPCD_ERR_CUDA, "cudaSetDevice failed"));
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(set_err(MPCD_ERR_CUDA, "stream"));
     const int n = c->n, Nc = c->Nc;
+    if ((rc = dalloc(&c->partFill, kPartBuckets))) return fail(rc);
     if (form == MPCD_FORM_FAST) {
         rc = fast_create(c, *params, device);
         if (rc) return fail(rc);
@@ -1549,21 +1593,20 @@ static int set_state_impl(mpcd_ctx* c, const double* x, const double* v, int64_t
     c->xflip = 0;
     c->slotsSorted = false;
     if (n > 0 && c->f32) {
-        // staged through FP64 scratch, then split into cell, FP32 offset and FP32 velocity
-        double2 *tx = nullptr, *tv = nullptr;
-        int rc = dalloc(&tx, (size_t)n);
-        if (!rc) rc = dalloc(&tv, (size_t)n);
-        if (!rc && (cudaMemcpyAsync(tx, x, sizeof(double2) * (size_t)n, kind, c->stream) != cudaSuccess ||
-                    cudaMemcpyAsync(tv, v, sizeof(double2) * (size_t)n, kind, c->stream) != cudaSuccess))
-            rc = set_err(MPCD_ERR_CUDA, "state upload");
-        if (!rc) {
-            k_f32_from<<<blocks_for(n), kThreads, 0, c->stream>>>(c->P, tx, tv, (int)n, view32(c, 0)); ++c->launches;
-            k_iota<<<blocks_for(n), kThreads, 0, c->stream>>>(c->pidb[0], (int)n); ++c->launches;
-            if (cudaStreamSynchronize(c->stream) != cudaSuccess) rc = set_err(MPCD_ERR_CUDA, "state conversion");
+        // split into cell, FP32 offset and FP32 velocity, from the caller's buffers where kernels
+        // may read them, else from a copy
+        const size_t bytes = sizeof(double2) * (size_t)n;
+        double2 *tx = f32_scratch_x(c), *tv = f32_scratch_v(c);
+        if (kind == cudaMemcpyDeviceToDevice && direct_device(x, bytes, c->device) && direct_device(v, bytes, c->device)) {
+            tx = (double2*)x;
+            tv = (double2*)v;
+        } else {
+            CUDA_TRY(cudaMemcpyAsync(tx, x, bytes, kind, c->stream));
+            CUDA_TRY(cudaMemcpyAsync(tv, v, bytes, kind, c->stream));
         }
-        cudaFree(tx);
-        cudaFree(tv);
-        if (rc) return rc;
+        k_f32_from<<<blocks_for(n), kThreads, 0, c->stream>>>(c->P, tx, tv, (int)n, view32(c, 0)); ++c->launches;
+        k_iota<<<blocks_for(n), kThreads, 0, c->stream>>>(c->pidb[0], (int)n); ++c->launches;
+        CUDA_TRY(cudaGetLastError());
     } else if (n > 0) {
         CUDA_TRY(cudaMemcpyAsync(c->xb[0], x, sizeof(double2) * (size_t)n, kind, c->stream));
         CUDA_TRY(cudaMemcpyAsync(c->vb[0], v, sizeof(double2) * (size_t)n, kind, c->stream));
@@ -1581,35 +1624,48 @@ int mpcd_set_state_device(mpcd_ctx* c, const double* x, const double* v, int64_t
     return set_state_impl(c, x, v, n, cudaMemcpyDeviceToDevice);
 }
 
+// the state into device buffers in particle-id order, enqueued on the context's stream (x, v
+// nullable; FP64: they may be the spare ping-pong buffers)
+static int store_state_async(mpcd_ctx* c, double2* x, double2* v) {
+    if (c->n == 0) return MPCD_OK;
+    double2 *sx = c->f32 ? nullptr : spare_x(c), *sv = c->f32 ? nullptr : c->vb[c->xv ^ 1];
+    if (c->f32) {
+        k_f32_by_pid<<<blocks_for(c->n), kThreads, 0, c->stream>>>(c->P, view32(c, c->xv), c->pidb[c->pp], c->n, x, v);
+    } else if (c->n >= kPartMin && x != sx && v != sv) {
+        // the intermediate arrays: the spare state buffers, and the key array for the ids
+        const PartBuf B{sx, sv, reinterpret_cast<int*>(c->sortKeys), c->partFill};
+        const int shift = part_shift(c->n);
+        CUDA_TRY(cudaMemsetAsync(c->partFill, 0, sizeof(int) * kPartBuckets, c->stream));
+        k_part_slots<<<blocks_for(c->n, kPartTile), kPartThreads, 0, c->stream>>>(cur_x(c), c->vb[c->xv], c->pidb[c->pp],
+                                                                                 c->n, shift, B);
+        k_part_place<<<blocks_for(c->n), 256, 0, c->stream>>>(B, c->n, shift, x, v);
+        ++c->launches;
+    } else {
+        k_gather_by_pid<<<blocks_for(c->n), kThreads, 0, c->stream>>>(cur_x(c), c->vb[c->xv], c->pidb[c->pp], c->n, x, v);
+    }
+    ++c->launches;
+    CUDA_TRY(cudaGetLastError());
+    return MPCD_OK;
+}
+
 static int get_state_impl(mpcd_ctx* c, double* x, double* v, bool toHost) {
     if (!c) return set_err(MPCD_ERR_INVALID_ARG, "null context");
     CUDA_TRY(cudaSetDevice(c->device));
     if (c->fast) return fast_get_state(c, x, v, toHost);
     if (c->n == 0) return MPCD_OK;
+    const size_t bytes = sizeof(double2) * (size_t)c->n;
+    // device buffers are written by the gather itself where kernels may write them; otherwise it
+    // goes through scratch that is free between calls (FP64: the other ping-pong buffers)
+    const bool apart = disjoint(x, v, bytes);
+    const bool dx = !toHost && x && apart && direct_device(x, bytes, c->device);
+    const bool dv = !toHost && v && apart && direct_device(v, bytes, c->device);
+    double2* tx = dx ? (double2*)x : (c->f32 ? f32_scratch_x(c) : spare_x(c));
+    double2* tv = dv ? (double2*)v : (c->f32 ? f32_scratch_v(c) : c->vb[c->xv ^ 1]);
+    int rc = store_state_async(c, x ? tx : nullptr, v ? tv : nullptr);
+    if (rc) return rc;
     const cudaMemcpyKind k = toHost ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
-    if (c->f32) {
-        double2 *tx = nullptr, *tv = nullptr;
-        int rc = dalloc(&tx, (size_t)c->n);
-        if (!rc) rc = dalloc(&tv, (size_t)c->n);
-        if (!rc) {
-            k_f32_by_pid<<<blocks_for(c->n), kThreads, 0, c->stream>>>(c->P, view32(c, c->xv), c->pidb[c->pp], c->n, tx, tv);
-            ++c->launches;
-            if ((x && cudaMemcpyAsync(x, tx, sizeof(double2) * (size_t)c->n, k, c->stream) != cudaSuccess) ||
-                (v && cudaMemcpyAsync(v, tv, sizeof(double2) * (size_t)c->n, k, c->stream) != cudaSuccess) ||
-                cudaStreamSynchronize(c->stream) != cudaSuccess)
-                rc = set_err(MPCD_ERR_CUDA, "state download");
-        }
-        cudaFree(tx);
-        cudaFree(tv);
-        if (rc) return rc;
-        return check_device(c);
-    }
-    double2* tx = spare_x(c);
-    double2* tv = c->vb[c->xv ^ 1];
-    k_gather_by_pid<<<blocks_for(c->n), kThreads, 0, c->stream>>>(cur_x(c), c->vb[c->xv], c->pidb[c->pp], c->n, tx, tv); ++c->launches;
-    CUDA_TRY(cudaGetLastError());
-    if (x) CUDA_TRY(cudaMemcpyAsync(x, tx, sizeof(double2) * (size_t)c->n, k, c->stream));
-    if (v) CUDA_TRY(cudaMemcpyAsync(v, tv, sizeof(double2) * (size_t)c->n, k, c->stream));
+    if (x && !dx) CUDA_TRY(cudaMemcpyAsync(x, tx, bytes, k, c->stream));
+    if (v && !dv) CUDA_TRY(cudaMemcpyAsync(v, tv, bytes, k, c->stream));
     return check_device(c);
 }
 
@@ -2418,19 +2474,6 @@ static int load_state_async(mpcd_ctx* c, const double2* x, const double2* v) {
         k_iota<<<blocks_for(c->n), kThreads, 0, c->stream>>>(c->pidb[0], c->n); ++c->launches;
     }
     invalidate_positions(c);
-    CUDA_TRY(cudaGetLastError());
-    return MPCD_OK;
-}
-
-// the state into device buffers in particle-id order, enqueued on the context's stream
-static int store_state_async(mpcd_ctx* c, double2* x, double2* v) {
-    if (c->n == 0) return MPCD_OK;
-    if (c->f32) {
-        k_f32_by_pid<<<blocks_for(c->n), kThreads, 0, c->stream>>>(c->P, view32(c, c->xv), c->pidb[c->pp], c->n, x, v);
-    } else {
-        k_gather_by_pid<<<blocks_for(c->n), kThreads, 0, c->stream>>>(cur_x(c), c->vb[c->xv], c->pidb[c->pp], c->n, x, v);
-    }
-    ++c->launches;
     CUDA_TRY(cudaGetLastError());
     return MPCD_OK;
 }

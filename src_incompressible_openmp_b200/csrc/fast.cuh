@@ -2036,7 +2036,11 @@ __global__ void k_fast_load(DevParams P, FastParams F, const double2* __restrict
     b.pid[s] = i;
 }
 
-// the bins into FP64 positions and velocities in particle-id order
+__device__ __forceinline__ double2 fast_position(const DevParams& P, int ix, int iy, float2 o) {
+    return make_double2(((double)ix + (double)o.x) * P.dx, ((double)iy + (double)o.y) * P.dy);
+}
+
+// the bins into FP64 positions and velocities in particle-id order (each nullable)
 __global__ void k_fast_store(DevParams P, FastParams F, FastBins b, double2* __restrict__ x, double2* __restrict__ v) {
     const int c = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -2049,8 +2053,8 @@ __global__ void k_fast_store(DevParams P, FastParams F, FastBins b, double2* __r
         if (p < 0 || p >= P.n) continue;
         const float2 o = b.off[s];
         const float2 w = b.vel[s];
-        x[p] = make_double2(((double)ix + (double)o.x) * P.dx, ((double)iy + (double)o.y) * P.dy);
-        v[p] = make_double2((double)w.x, (double)w.y);
+        if (x) x[p] = fast_position(P, ix, iy, o);
+        if (v) v[p] = make_double2((double)w.x, (double)w.y);
     }
 }
 
