@@ -517,6 +517,40 @@ int validate(const mpcd_params_c& p) {
     return MPCD_OK;
 }
 
+// DevParams::zt from the thresholds (src/zone_pass.cpp:321-366) and the angular bins
+void zone_tables(DevParams& d) {
+    ZoneTables& z = d.zt;
+    z = ZoneTables{};
+    if (d.useLFF) return;
+    // empty cells: fluid fraction 1 (map_low and map_high of zone.cuh without local fractions)
+    const double thr[2][2] = {{std::max(d.lowFrac * d.gamma, d.lowThrFloor), d.lowThrBulk},
+                              {std::max(d.highFrac * d.gamma, d.highThrFloor), d.highThr}};
+    for (int m = 0; m < 2; ++m)
+        for (int k = 0; k < 2; ++k) {
+            if (!(thr[m][k] >= 1.0 && thr[m][k] <= 127.0)) return;
+            z.cut[m][k] = (int)std::ceil(thr[m][k]);
+            z.flo[m][k] = (int)std::floor(thr[m][k]);
+        }
+    for (int m = 0; m < 2; ++m) {
+        const double f0 = thr[m][0] - std::floor(thr[m][0]), f1 = thr[m][1] - std::floor(thr[m][1]);
+        z.up[m][0] = f0 > f1;
+        z.up[m][1] = f1 > f0;
+    }
+    z.highThr[0] = thr[1][0];
+    z.highThr[1] = thr[1][1];
+    int fill[8] = {};
+    for (int kk = 0; kk < 25; ++kk) {
+        if (kk == 12) continue;
+        const int dy = kk / 5 - 2, dx = kk % 5 - 2, b = d.atanBin[(dx + 2) + 5 * (dy + 2)];
+        if (fill[b] >= 3) return;
+        const int lane = 3 * b + fill[b]++;
+        z.dx[lane] = (signed char)dx;
+        z.dy[lane] = (signed char)dy;
+        z.orig[lane] = (unsigned char)(kk < 12 ? kk : kk - 1);
+    }
+    z.ok = 1;
+}
+
 // Host-side derived constants; libm values where the reference calls libm.
 DevParams make_dev_params(const mpcd_params_c& p) {
     DevParams d{};
@@ -576,6 +610,7 @@ DevParams make_dev_params(const mpcd_params_c& p) {
             d.atanBin[(a + 2) + 5 * (b + 2)] = ib;
             d.hypotTab[(a + 2) + 5 * (b + 2)] = std::hypot((double)a, (double)b);
         }
+    zone_tables(d);
     return d;
 }
 
@@ -1517,15 +1552,22 @@ int mpcd_ctx_create_form(const mpcd_params_c* params, int device, int32_t form, 
             !raise_smem((const void*)k_zone_pass<true>, c->zSmem, device) ||
             !raise_smem((const void*)k_zone_serial, c->zSmem, device))
             return fail(set_err(MPCD_ERR_CUDA, "zone shared memory attribute"));
-        // the phase-synchronous kernel: the most warps per block (16, 8 or 4) whose working
-        // sets fit in 200 KB; MPCD_ZONE_SYNC_WARPS picks another (0: one zone per block)
+        // Zones per block, run in step (k_zone_pass_sync), from the zones of a pass. With few of them
+        // the pass is one zone's latency, and zones that share an SM only slow each other: one zone
+        // per block up to 4 per SM. With more, zones in step share the instruction cache, and wider
+        // blocks pay once there are waves of them. Measured (zone phases of a step, ms, for W = 0, 4,
+        // 8, 16): 25 zones 0.233 0.241 0.256 0.281; 340: 0.264 0.271 0.285 0.314; 800: 0.357 0.306
+        // 0.316 0.341; 1,352: 0.416 0.338 0.331 0.334; 5,356: 1.000 0.870 0.823 0.868; 10,660: 2.525
+        // 1.928 1.548 1.501. W working sets must fit in 200 KB. MPCD_ZONE_SYNC_WARPS picks another
+        // (0: one zone per block).
         c->zSyncWarps = 0;
-        if (c->zMaxCells > 0)
-            for (int W : {16, 8, 4})
-                if ((size_t)W * c->zSmem <= 200 * 1024) {
-                    c->zSyncWarps = W;
-                    break;
-                }
+        if (c->zMaxCells > 0) {
+            constexpr int kSms = 148;
+            const int nz = std::max(B.nZones, S.nZones);
+            int W = nz <= 4 * kSms ? 0 : (nz <= 8 * kSms ? 4 : (nz <= 64 * kSms ? 8 : 16));
+            while (W > 0 && (size_t)W * c->zSmem > 200 * 1024) W = W > 4 ? W / 2 : 0;
+            c->zSyncWarps = W;
+        }
         if (const char* e = std::getenv("MPCD_ZONE_SYNC_WARPS")) {
             const int v = std::atoi(e);
             if ((v == 0 || v == 4 || v == 8 || v == 16) && (size_t)v * c->zSmem <= 200 * 1024) c->zSyncWarps = v;

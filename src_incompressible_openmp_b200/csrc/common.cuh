@@ -43,6 +43,21 @@ __device__ __forceinline__ void raise_error(DevStatus* st, int code, int detail)
     if (atomicCAS(&st->code, 0, code) == 0) st->detail = detail;
 }
 
+// Integer forms of the zone pass's thresholds and of its 24 range-2 neighbours, for the parameter
+// sets that have them (host: zone_tables in capi.cu). thr[map][cls]: map 0 low, 1 high; cls 1 for
+// cells that were occupied when the maps were built, 0 for the others. For an integer count n,
+//   n < thr  <=>  n < cut,    n > thr  <=>  n > flo,    floor(thr - n) = flo - n  (n <= thr).
+// The deficits thr - n of two cells compare like 2 (flo - n) + up: up ranks the fractional parts.
+struct ZoneTables {
+    int ok;              // 0: local fluid fractions, thresholds outside [1, 127], or an angular bin
+                         // without exactly three neighbours: the general routines run
+    int cut[2][2], flo[2][2], up[2][2];
+    double highThr[2];   // thr[1][cls]
+    // neighbours grouped by angular bin: lane 3 b + k holds the k-th of bin b
+    signed char dx[24], dy[24];
+    unsigned char orig[24];  // its place in the reference's scan order (dy outer, dx inner)
+};
+
 // Parameter block passed by value to every kernel. Derived constants are computed on the
 // host once per context, with the host libm where the reference calls libm (cos, sin,
 // atan2 and hypot of small integer steps).
@@ -66,6 +81,7 @@ struct DevParams {
     double hypotTab[25];
     // FP32 precision form: the largest FP32 offsets strictly inside a cell (x, y)
     float offMaxX, offMaxY;
+    ZoneTables zt;
 };
 
 // Device-side seed table of one step (CUDA-graph replay: the step number lives on the

@@ -115,7 +115,7 @@ struct ZoneMem {
     uint16_t* order;   // cell: arena order of materialised lists (compaction)
     uint32_t* arena;   // arenaCap
     int* small;        // 64 ints: ranked targets, donors
-    double* smallD;    // 24 doubles: donor normals, their polar components and radii
+    double* smallD;    // 16 doubles: the donors' deviates, polar components and radii
 
     __host__ __device__ static size_t bytes(int maxCells, int winCap, int arenaCap, int nsmCap) {
         size_t b = 0;
@@ -131,7 +131,7 @@ struct ZoneMem {
         add((size_t)maxCells * 2, 2);
         add((size_t)arenaCap * 4, 4);
         add(64 * 4, 4);
-        add(24 * 8, 8);
+        add(16 * 8, 8);
         return (b + 15) / 16 * 16;
     }
     __device__ void carve(char* base, int maxCells, int winCap, int arenaCap, int nsmCap) {
@@ -157,7 +157,7 @@ struct ZoneMem {
         order = (uint16_t*)take((size_t)maxCells * 2, 2);
         arena = (uint32_t*)take((size_t)arenaCap * 4, 4);
         small = (int*)take(64 * 4, 4);
-        smallD = (double*)take(24 * 8, 8);
+        smallD = (double*)take(16 * 8, 8);
     }
 };
 
@@ -358,11 +358,15 @@ __device__ __forceinline__ void zone_shuffle_fast(T* a, int m, ZoneMt& r, int la
         return;
     }
     r.consume(D);
+    // draw k swaps entry i_k (known from k) with p1 and entry i_k + 1 with p2: one shuffle fetches
+    // both places, two move the values
     unsigned v = (lane < m) ? (unsigned)a[lane] : 0u;
+    const int pq = p1 | (p2 << 8);  // p2 = -1: no second swap
+    const int i0 = even ? 2 : 1;
     for (int k = 0; k < D; ++k) {
-        const int ik = __shfl_sync(0xffffffffu, i, k);
-        const int a1 = __shfl_sync(0xffffffffu, p1, k);
-        const int a2 = __shfl_sync(0xffffffffu, p2, k);
+        const int w = __shfl_sync(0xffffffffu, pq, k);
+        const int a1 = w & 0xff, a2 = w >> 8;
+        const int ik = (even && k == 0) ? 1 : i0 + 2 * (k - (even ? 1 : 0));
         v = __shfl_sync(0xffffffffu, v, (lane == ik) ? a1 : ((lane == a1) ? ik : lane));
         if (a2 >= 0) {
             const int i2 = ik + 1;
@@ -479,16 +483,25 @@ __device__ __noinline__ void zone_compute_nsm(double* nsm, const W* win, const I
     __syncwarp();
 }
 
-// hypot, out of line (once per sparse cell)
-__device__ __noinline__ double zone_hypot(double a, double b) { return mpcd_dd::hypot_cr(a, b); }
+// A donor's score 100 align + Nsm + 1e-9 N(0,1) with the correctly rounded norm of the gradient
+// and deviate (comp, rad: zone_normals_draw), the reference's value. Out of line: it runs only
+// where the ranking is not certain without it.
+__device__ __noinline__ double zone_exact_score(double gx, double gy, double ddx, double ddy, double nstep, double nsmd,
+                                                double comp, double rad) {
+    const double ndir = mpcd_dd::hypot_cr(gx, gy);
+    double align = 0.0;
+    if (ndir >= 1e-14 && nstep >= 1e-14)
+        align = __ddiv_rn(__dadd_rn(__dmul_rn(ddx, gx), __dmul_rn(ddy, gy)), __dmul_rn(ndir, nstep));
+    const double noise = __dmul_rn(1e-9, __dmul_rn(comp, polar_scale(rad)));
+    return __dadd_rn(__dadd_rn(__dmul_rn(100.0, align), nsmd), noise);
+}
 
 // cnt deviates of one fresh normal_distribution (polar method: pairs of uniforms in stream
-// order until r2 is in (0, 1]; each accepted pair gives y*m, then the cached x*m) into out[].
-// Lane c examines candidate pair c of the batch; the accepted ones are ranked by ballot. The
-// polar scale m uses the CUDA log (a few ulp from the correctly rounded one); comp and rad
-// keep each deviate's polar component and r2, so that the exact deviate can be rebuilt as
-// comp * polar_scale(r2).
-__device__ __forceinline__ void zone_normals_fast(double* out, double* comp, double* rad, int cnt, ZoneMt& r, int lane) {
+// order until r2 is in (0, 1]; each accepted pair gives y*m, then the cached x*m), drawn but not
+// evaluated: comp and rad receive each deviate's polar component and r2, so that the deviate is
+// comp * polar_scale(r2). Lane c examines candidate pair c of the batch; the accepted ones are
+// ranked by ballot.
+__device__ __forceinline__ void zone_normals_draw(double* comp, double* rad, int cnt, ZoneMt& r, int lane) {
     int got = 0;
     while (got < cnt) {
         r.ensure(2 * kWarp);
@@ -503,13 +516,10 @@ __device__ __forceinline__ void zone_normals_fast(double* out, double* comp, dou
         int last = kWarp - 1;
         if (__popc(am) >= need) last = __ffs(__ballot_sync(0xffffffffu, acc && rank == need - 1)) - 1;
         if (acc && rank < need) {
-            const double mult = sqrt(__ddiv_rn(__dmul_rn(-2.0, log(r2)), r2));
             const int k0 = got + 2 * rank;
-            out[k0] = __dmul_rn(y, mult);
             comp[k0] = y;
             rad[k0] = r2;
             if (k0 + 1 < cnt) {
-                out[k0 + 1] = __dmul_rn(x, mult);
                 comp[k0 + 1] = x;
                 rad[k0 + 1] = r2;
             }
@@ -536,6 +546,10 @@ struct ZoneState {
     int atanLane;   // lane k < 25 holds the angular bin of step k (DevParams::atanBin)
     double hypLane; // lane k < 25 holds the length of step k (DevParams::hypotTab)
     bool nbDirect;  // no wrapped neighbour (|offset| <= 2) of a zone cell lies in the zone
+    // dense cells by the integer tables (dense_cell_fast): this lane's range-2 neighbour as an
+    // offset of the local cell, its step (dx, dy), scan place, and (chebyshev << 4 | distance^2)
+    bool fast;
+    int nOff, nDx, nDy, nOrig, nKey;
     bool dupNb5;    // a periodic axis shorter than 5 cells: range-2 neighbours can coincide
     bool dupNb3;    // a periodic axis shorter than 3 cells: 8-neighbours can coincide
     bool failed;   // capacity exhausted: the zone is handed to the overflow path
@@ -917,20 +931,172 @@ struct ZoneState {
         movedDense += moved;
     }
 
-    // ------------------------------------------------------------------ sparse phase
-    __device__ void inward(int l, double& gx, double& gy) const {
+    // One dense cell, as dense_cell, for zones whose tables hold (fast). Lane 3 b + k examines the
+    // k-th neighbour of angular bin b for the whole call: the ranking compares a lane with the two
+    // others of its bin, and counts order by ballots over (rank, bin) instead of loops over the
+    // bins. All sums and comparisons are on integers (ZoneTables); the tie draw of a target is
+    // consumed but never read, since the neighbours of a bin differ in (chebyshev, distance^2).
+    // When no more particles leave than targets have a deficit, the round robin's quota stays 1:
+    // the first `need` of them take one particle each, in one step with a lane per move (the usual
+    // case; the general loop handles the rest). Bound by the latency of its dependent
+    // instructions: a call takes 4,300 cycles with one zone per SM (8,600 in the general form),
+    // 7,200 with 16 (12,500).
+    __device__ void dense_cell_fast(int l) {
         const DevParams& p = P();
-        const int ix = gx_of(l), iy = gy_of(l);
-#define NS(jx, jy) M.nsm[nsm_index((jx), (jy))]
-        if (p.perx) gx = __dmul_rn(0.5, __dsub_rn(NS(wrap_index(ix + 1, p.Nx), iy), NS(wrap_index(ix - 1, p.Nx), iy)));
-        else if (ix == 0) gx = __dsub_rn(NS(ix + 1, iy), NS(ix, iy));
-        else if (ix == p.Nx - 1) gx = __dsub_rn(NS(ix, iy), NS(ix - 1, iy));
-        else gx = __dmul_rn(0.5, __dsub_rn(NS(ix + 1, iy), NS(ix - 1, iy)));
-        if (p.pery) gy = __dmul_rn(0.5, __dsub_rn(NS(ix, wrap_index(iy + 1, p.Ny)), NS(ix, wrap_index(iy - 1, p.Ny))));
-        else if (iy == 0) gy = __dsub_rn(NS(ix, iy + 1), NS(ix, iy));
-        else if (iy == p.Ny - 1) gy = __dsub_rn(NS(ix, iy), NS(ix, iy - 1));
-        else gy = __dmul_rn(0.5, __dsub_rn(NS(ix, iy + 1), NS(ix, iy - 1)));
-#undef NS
+        const ZoneTables& z = p.zt;
+        const int sCls = (M.cflags[l] & kCBulkBefore) ? 1 : 0;
+        const int sFlo = z.flo[1][sCls];
+        const int len0 = M.len[l];
+        if (len0 <= sFlo) return;
+        // ceil(n - high) in FP64, as an integer where the subtraction is exact
+        auto excess = [&](int n) {
+            return n <= 2 * sFlo ? max(0, n - sFlo) : (int)ceil(__dsub_rn((double)n, z.highThr[sCls]));
+        };
+        const int lx = lx_of(l), ly = l - lx * TY;
+        const int t = l + nOff;
+        const bool in = lane < 24 && (unsigned)(lx + nDx) < (unsigned)TX && (unsigned)(ly + nDy) < (unsigned)TY;
+        // the slots of the owned entries that may leave, loaded ahead
+        int slotPre = -1;
+        if (lane < min(len0, excess(len0))) {
+            const uint32_t e = elem(l, lane);
+            const int lc = (int)(e >> kEntryShift);
+            if (M.cflags[lc] & kCOwned) slotPre = A->slots[M.gstart[lc] + (int)(e & ((1u << kEntryShift) - 1))];
+        }
+        const int tCls = (in && (M.cflags[t] & kCBulkBefore)) ? 1 : 0;
+        const int bin = lane / 3, base = 3 * bin;
+        bool recv = false;
+        int moved = 0;
+#pragma unroll 1
+        for (int round = 0; round < 2; ++round) {
+            const int need = excess(len0 - moved);
+            if (need <= 0) break;
+            const int tLen = in ? M.len[t] : 0;
+            const bool adm = in && tLen < z.cut[round][tCls];
+            const unsigned om = __reduce_or_sync(0xffffffffu, adm ? (1u << nOrig) : 0u);
+            if (om == 0) continue;
+            const int m = __popc(om);
+            rng.ensure(m + 1);
+            const int startBin = (int)(rng.peek(0) >> 61);  // uniform_int(1, 8) - 1
+            rng.consume(m + 1);
+            // rank within the bin on (-deficit, cnt, chebyshev, distance^2)
+            const int def = z.flo[round][tCls] - tLen;
+            const unsigned key =
+                adm ? ((unsigned)(255 - (2 * def + z.up[round][tCls])) << 13) | ((unsigned)tLen << 6) | (unsigned)nKey
+                    : 0xffffffffu;
+            const unsigned ka = __shfl_sync(0xffffffffu, key, base + (lane - base + 1) % 3);
+            const unsigned kb = __shfl_sync(0xffffffffu, key, base + (lane - base + 2) % 3);
+            // place in the round robin: rank, then bin from the start bin on
+            const int q = ((ka < key) + (kb < key)) * 8 + ((bin - startBin) & 7);
+            const unsigned below = (1u << (q & 31)) - 1u;
+            const unsigned pm = __reduce_or_sync(0xffffffffu, adm && def > 0 ? (1u << q) : 0u);
+            if (pm == 0) continue;
+            bool one = need <= __popc(pm);
+            const int i = __popc(pm & below);  // this target's turn
+            const bool act = one && adm && def > 0 && i < need;
+            int dst = 0;
+            if (one) {
+                // room for one entry at the end of each receiving list
+                bool grow = act;
+                if (act && (M.cflags[t] & kCMat)) {
+                    const int hd = M.head[t];
+                    dst = M.abase[t] + hd + tLen;
+                    grow = hd + tLen >= (int)M.cap[t];
+                }
+                if (__any_sync(0xffffffffu, grow)) {
+                    const int want = grow ? tLen + 5 : 0;
+                    int end = want;
+#pragma unroll
+                    for (int o = 1; o < kWarp; o <<= 1) {
+                        const int u = __shfl_up_sync(0xffffffffu, end, o);
+                        if (lane >= o) end += u;
+                    }
+                    const int total = __shfl_sync(0xffffffffu, end, kWarp - 1);
+                    one = arenaTop + total <= arenaCap;
+                    if (one && grow) {
+                        const int a = arenaTop + end - want;
+                        const bool mat = (M.cflags[t] & kCMat) != 0;
+                        const int from = M.head[t] + (mat ? (int)M.abase[t] : 0);
+                        const uint32_t e0 = ((uint32_t)t << kEntryShift) | (uint32_t)from;
+                        for (int j = 0; j < tLen; ++j) M.arena[a + j] = mat ? M.arena[from + j] : e0 + (uint32_t)j;
+                        M.abase[t] = a;
+                        M.head[t] = 0;
+                        M.cap[t] = want;
+                        M.cflags[t] |= kCMat;
+                        dst = a + tLen;
+                    }
+                    if (one) arenaTop += total;
+                    __syncwarp();
+                }
+            }
+            if (!one) {
+                int* T = M.small;
+                const unsigned am = __reduce_or_sync(0xffffffffu, adm ? (1u << q) : 0u);
+                if (adm) T[__popc(am & below)] = t;
+                __syncwarp();
+                int recvReg = -1, nrecv = 0;
+                moved += spread(l, T, m, round == 0, need, recvReg, nrecv, slotPre, moved);
+                if (failed || fatal) return;
+                for (int k = 0; k < nrecv; ++k)
+                    if (__shfl_sync(0xffffffffu, recvReg, k) == t && in) recv = true;
+                continue;
+            }
+            rng.ensure(2 * need);
+            const int w = moved + i;
+            const int pre = __shfl_sync(0xffffffffu, slotPre, w & (kWarp - 1));
+            if (act) {
+                const uint32_t e = elem(l, i);
+                const double px = __dadd_rn(__dmul_rn((double)(xs + lx + nDx), p.dx), __dmul_rn(p.dx, canon(rng.peek(2 * i))));
+                const double py = __dadd_rn(__dmul_rn((double)(ys + ly + nDy), p.dy), __dmul_rn(p.dy, canon(rng.peek(2 * i + 1))));
+                const int lc = (int)(e >> kEntryShift);
+                if (M.cflags[lc] & kCOwned) {
+                    const int sl = (w < kWarp) ? pre : A->slots[M.gstart[lc] + (int)(e & ((1u << kEntryShift) - 1))];
+                    const int cc = cell_of(px, py, p);
+                    if (kF32)
+                        A->out32.set_pos(sl, make_double2(px, py), cc, p);
+                    else
+                        A->xout[sl] = make_double2(px, py);
+                    A->cid[sl] = cc;
+                }
+                M.arena[dst] = e;
+                M.len[t] = tLen + 1;
+                recv = true;
+            }
+            rng.consume(2 * need);
+            moved += need;
+            __syncwarp();
+            if (lane == 0) {
+                M.head[l] += need;
+                M.len[l] -= need;
+            }
+            __syncwarp();
+        }
+        // receivers' flags and update_transfer_correction_masks (src/zone_pass.cpp:492-525) on the
+        // source (lane 31) and its receivers
+        const bool allBulk = sCls && __all_sync(0xffffffffu, !recv || tCls);
+        if (recv || lane == kWarp - 1) {
+            const int c = recv ? t : l;
+            uint8_t f = M.cflags[c];
+            if (recv) f |= kCRecv | kCChanged;
+            else if (moved > 0) f |= kCChanged;
+            M.cflags[c] = allBulk ? (uint8_t)(f | kCBulkBulk) : (uint8_t)((f | kCSkip) & ~kCBulkBulk);
+        }
+        __syncwarp();
+        movedDense += moved;
+    }
+
+    // ------------------------------------------------------------------ sparse phase
+    // Gradient of the smoothed occupancy at cell l (src/zone_pass.cpp:375-411). The ring around the
+    // zone holds the wrapped neighbours' values, so the map is read at local offsets.
+    __device__ __forceinline__ void inward(int l, int at, double& gx, double& gy) const {
+        const DevParams& p = P();
+        const int ix = gx_of(l), iy = gy_of(l), SY = TY + 2;
+        const double* n = M.nsm + at;
+        if (!p.perx && ix == 0) gx = __dsub_rn(n[SY], n[0]);
+        else if (!p.perx && ix == p.Nx - 1) gx = __dsub_rn(n[0], n[-SY]);
+        else gx = __dmul_rn(0.5, __dsub_rn(n[SY], n[-SY]));
+        if (!p.pery && iy == 0) gy = __dsub_rn(n[1], n[0]);
+        else if (!p.pery && iy == p.Ny - 1) gy = __dsub_rn(n[0], n[-1]);
+        else gy = __dmul_rn(0.5, __dsub_rn(n[1], n[-1]));
     }
 
     // one sparse cell (src/zone_pass.cpp:804-854)
@@ -939,15 +1105,18 @@ struct ZoneState {
         int* don = M.small + 32;
         const int ncc = M.len[l];
         if (ncc <= 0) return;
-        if (M.len[l] == 0) return;
-        const int ix = gx_of(l), iy = gy_of(l);
+        const int lx = lx_of(l), ly = l - lx * TY;
+        const int ix = xs + lx, iy = ys + ly;
         int nb = -1;
         if (lane < 8) {
             const int kk = (lane < 4) ? lane : lane + 1;
             const int dy = kk / 3 - 1, dx = kk % 3 - 1;
-            int jy, jx;
-            if (nbDirect ? in_zone(jx = ix + dx, jy = iy + dy) : (shift_index(iy, ix, dy, dx, jy, jx) && in_zone(jx, jy)))
-                nb = loc(jx, jy);
+            if (nbDirect) {
+                if ((unsigned)(lx + dx) < (unsigned)TX && (unsigned)(ly + dy) < (unsigned)TY) nb = l + dx * TY + dy;
+            } else {
+                int jy, jx;
+                if (shift_index(iy, ix, dy, dx, jy, jx) && in_zone(jx, jy)) nb = loc(jx, jy);
+            }
         }
         const unsigned m0 = __ballot_sync(0xffffffffu, nb >= 0);
         if (m0 == 0) return;
@@ -965,48 +1134,51 @@ struct ZoneState {
         if (nd == 0) return;
         if (isDonor) don[__popc(md & lanemask_lt())] = nb;
         __syncwarp();
-        double gx, gy;
-        inward(l, gx, gy);
         zone_shuffle_fast(don, nd, rng, lane);
-        // one N(0,1) per donor in shuffled order, then scores in parallel (lane k = donor k).
-        // The scores only rank the donors: they are computed first with the CUDA hypot and
-        // log, and again with the correctly rounded ones (the reference's values) only if two
-        // scores lie closer than those functions' few-ulp differences could move them.
-        double* nrm = M.smallD;
-        zone_normals_fast(nrm, M.smallD + 8, M.smallD + 16, nd, rng, lane);
+        // One N(0,1) per donor in shuffled order, then scores in parallel (lane k = donor k). The
+        // score 100 align + Nsm + 1e-9 N(0,1) only ranks the donors, and |N(0,1)| stays below 12
+        // (r2 >= 2^-106), so the deviates and the last bits of the norm matter only where two
+        // scores lie within 3e-8 of each other: the scores come from sqrt(gx^2 + gy^2) (within
+        // 1e-12 (1 + |score|) of the reference's) without the deviates, and a ranking with a gap of
+        // 1e-7 (1 + |score|) or less between two donors is done again from the exact values.
+        zone_normals_draw(M.smallD, M.smallD + 8, nd, rng, lane);
+        const int SY = TY + 2, at = (lx + 1) * SY + ly + 1;
+        double gx, gy;
+        inward(l, at, gx, gy);
         int dk = -1, idx = 0, ddx = 0, ddy = 0;
+        double nsmd = 0.0;
         if (lane < nd) {
             dk = don[lane];
-            idx = step_index(ix, iy, gx_of(dk), gy_of(dk), ddx, ddy);
+            const int dlx = lx_of(dk), dly = dk - dlx * TY;
+            idx = step_index(ix, iy, xs + dlx, ys + dly, ddx, ddy);
+            nsmd = M.nsm[(dlx + 1) * SY + dly + 1];
         }
         const double hs = __shfl_sync(0xffffffffu, hypLane, idx < 0 ? 0 : idx);
-        const double nsmd = (lane < nd) ? M.nsm[nsm_index(gx_of(dk), gy_of(dk))] : 0.0;
-        auto score = [&](double ndir, double nv) {
-            const double nstep = (idx >= 0) ? hs : 0.0;
-            double align = 0.0;
-            if (ndir >= 1e-14 && nstep >= 1e-14)
-                align = __ddiv_rn(__dadd_rn(__dmul_rn((double)ddx, gx), __dmul_rn((double)ddy, gy)), __dmul_rn(ndir, nstep));
-            const double noise = __dmul_rn(1e-9, nv);
-            return __dadd_rn(__dadd_rn(__dmul_rn(100.0, align), nsmd), noise);
-        };
-        const double ndirF = hypot(gx, gy);
-        double sc = (lane < nd) ? score(ndirF, nrm[lane]) : 0.0;
-        // the fast and exact scores differ by under 2e-13 (1 + |score|): distinct ranks are
-        // certain when every gap exceeds 1e-12 (1 + |score|) and the norm is clear of 1e-14
+        const double nstep = (idx >= 0) ? hs : 0.0;
+        const double ndirF = sqrt(__dadd_rn(__dmul_rn(gx, gx), __dmul_rn(gy, gy)));
+        double sc = 0.0;
+        if (lane < nd && ndirF >= 1e-14 && nstep >= 1e-14)
+            sc = __dmul_rn(100.0, __ddiv_rn(__dadd_rn(__dmul_rn((double)ddx, gx), __dmul_rn((double)ddy, gy)),
+                                            __dmul_rn(ndirF, nstep)));
+        sc = __dadd_rn(sc, nsmd);
         bool sure = !(ndirF > 0.5e-14 && ndirF < 2e-14);
+        int rk = 0;  // descending
         for (int j = 0; j < nd; ++j) {
             const double sj = __shfl_sync(0xffffffffu, sc, j);
-            if (lane < nd && j != lane && fabs(sj - sc) <= 1e-12 * (1.0 + fabs(sc))) sure = false;
+            if (lane < nd && j != lane) {
+                if (fabs(sj - sc) <= 1e-7 * (1.0 + fabs(sc))) sure = false;
+                rk += sj > sc;
+            }
         }
         if (!__all_sync(0xffffffffu, sure)) {
-            const double ndir = zone_hypot(gx, gy);
-            if (lane < nd) sc = score(ndir, __dmul_rn(M.smallD[8 + lane], polar_scale(M.smallD[16 + lane])));
-        }
-        // descending, ties in shuffled order (std::sort of <= 16 elements is an insertion sort)
-        int rk = 0;
-        for (int j = 0; j < nd; ++j) {
-            const double sj = __shfl_sync(0xffffffffu, sc, j);
-            if (lane < nd && j != lane && (sj > sc || (sj == sc && j < lane))) ++rk;
+            sc = 0.0;
+            if (lane < nd)
+                sc = zone_exact_score(gx, gy, (double)ddx, (double)ddy, nstep, nsmd, M.smallD[lane], M.smallD[8 + lane]);
+            rk = 0;  // ties in shuffled order (std::sort of <= 16 elements is an insertion sort)
+            for (int j = 0; j < nd; ++j) {
+                const double sj = __shfl_sync(0xffffffffu, sc, j);
+                if (lane < nd && j != lane && (sj > sc || (sj == sc && j < lane))) ++rk;
+            }
         }
         __syncwarp();
         if (lane < nd) don[rk] = dk;
@@ -1135,6 +1307,15 @@ __device__ __forceinline__ bool zone_setup(ZoneState<I, kF32>& S, const ZoneArgs
     S.dupNb5 = (p.perx && p.Nx < 5) || (p.pery && p.Ny < 5);
     S.nbDirect = (!p.perx || S.TX < p.Nx - 2) && (!p.pery || S.TY < p.Ny - 2);
     S.dupNb3 = (p.perx && p.Nx < 3) || (p.pery && p.Ny < 3);
+    S.fast = p.zt.ok && S.nbDirect;
+    S.nDx = S.nDy = S.nOff = S.nOrig = S.nKey = 0;
+    if (lane < 24) {
+        S.nDx = p.zt.dx[lane];
+        S.nDy = p.zt.dy[lane];
+        S.nOrig = p.zt.orig[lane];
+        S.nOff = S.nDx * S.TY + S.nDy;
+        S.nKey = (max(abs(S.nDx), abs(S.nDy)) << 4) | (S.nDx * S.nDx + S.nDy * S.nDy);
+    }
     const int W = (S.TX + 4) * S.WY;
     if (S.nl > maxCells || W > winCap || (S.TX + 2) * (S.TY + 2) > nsmCap || S.nl >= (1 << (32 - kEntryShift)) ||
         (sizeof(I) == 2 && S.nl > 65535))
@@ -1220,9 +1401,15 @@ __device__ __forceinline__ int zone_dense_pass(ZoneState<I, kF32>& S) {
     ZoneMem<I>& M = S.M;
     if (p.useLFF) S.compute_nsm();
     S.mark_bulk();
-    const int nd = S.collect([&](int l) { return (double)M.len[l] > S.map_high(l); });
+    const int nd = S.collect([&](int l) {
+        return S.fast ? (int)M.len[l] > p.zt.flo[1][(M.cflags[l] & kCBulkBefore) ? 1 : 0]
+                      : (double)M.len[l] > S.map_high(l);
+    });
     zone_shuffle_fast(M.list, nd, S.rng, lane);
-    for (int q = 0; q < nd && !S.failed && !S.fatal; ++q) S.dense_cell((int)M.list[q]);
+    for (int q = 0; q < nd && !S.failed && !S.fatal; ++q) {
+        if (S.fast) S.dense_cell_fast((int)M.list[q]);
+        else S.dense_cell((int)M.list[q]);
+    }
     return nd;
 }
 
@@ -1261,11 +1448,10 @@ __device__ __forceinline__ bool zone_finish(ZoneState<I, kF32>& S, const ZoneArg
     double dgUx2 = 0.0, dgUy2 = 0.0, dgPx2 = 0.0, dgPy2 = 0.0;
     int dgNPx = 0, dgNPy = 0;
     for (int l = lane; l < S.nl; l += kWarp) {
-        double d2 = 0.0;
-        const uint8_t f = M.cflags[l];
-        const int n = M.len[l];
+        du2[l] = 0.0;
         if (kSerial) A.duScratch[l] = make_double2(0.0, 0.0);  // cells left unchanged get none
-        if (wantDiag && !(f & kCChanged) && n > 0) {
+        const int n = M.len[l];
+        if (wantDiag && !(M.cflags[l] & kCChanged) && n > 0) {
             // an unchanged cell: uxNow from its input list (ascending id), no momentum error
             double sx = 0.0, sy = 0.0;
             for (int j = 0; j < n; ++j) {
@@ -1277,73 +1463,83 @@ __device__ __forceinline__ bool zone_finish(ZoneState<I, kF32>& S, const ZoneArg
             dgUx2 = __dadd_rn(dgUx2, __dmul_rn(ux, ux));
             dgUy2 = __dadd_rn(dgUy2, __dmul_rn(uy, uy));
         }
-        if ((f & kCChanged) && n > 0) {
-            double bx = 0.0, by = 0.0, axs = 0.0, ays = 0.0;
-            const int n0 = M.cnt0[l], g0 = M.gstart[l];
-            for (int j0 = 0; j0 < n0; j0 += 8) {
-                int sl[8];
-                double2 w[8];
+    }
+    // The changed cells, one per lane (listed first: about 70 of a base zone's 100, few of a
+    // shifted one's). A lane's chain is slot, then velocity, for each of its
+    // particles; the slots of 16 are loaded together, then their velocities in two batches of 8.
+    // A materialised list is dead after its sum: its entries are replaced by their slots there
+    // (bit 31: not owned), so that the correction finds them without another look-up.
+    constexpr int kOwnBit = (int)0x80000000u;
+    const int nch = S.collect([&](int l) { return (M.cflags[l] & kCChanged) && M.len[l] > 0; });
+    for (int q = lane; q < nch; q += kWarp) {
+        const int l = M.list[q];
+        const uint8_t f = M.cflags[l];
+        const int n = M.len[l], g0 = M.gstart[l];
+        const bool mat = (f & kCMat) != 0;
+        const int at = (mat ? (int)M.abase[l] : g0) + (int)M.head[l];
+        auto sum = [&](int cnt, auto slotAt, double& sx, double& sy) {
+            for (int j0 = 0; j0 < cnt; j0 += 16) {
+                int sl[16];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) sl[u] = (j0 + u < n0) ? A.slots[g0 + j0 + u] : 0;
+                for (int u = 0; u < 16; ++u) sl[u] = (j0 + u < cnt) ? slotAt(j0 + u) : 0;
 #pragma unroll
-                for (int u = 0; u < 8; ++u) w[u] = (j0 + u < n0) ? zone_vin<kF32>(A, sl[u]) : make_double2(0.0, 0.0);
+                for (int h = 0; h < 16; h += 8) {
+                    if (j0 + h >= cnt) break;
+                    double2 w[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (j0 + u < n0) {
-                        bx = __dadd_rn(bx, w[u].x);
-                        by = __dadd_rn(by, w[u].y);
-                    }
+                    for (int u = 0; u < 8; ++u) w[u] = (j0 + h + u < cnt) ? zone_vin<kF32>(A, sl[h + u]) : make_double2(0.0, 0.0);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (j0 + h + u < cnt) {
+                            sx = __dadd_rn(sx, w[u].x);
+                            sy = __dadd_rn(sy, w[u].y);
+                        }
+                }
             }
+        };
+        double bx = 0.0, by = 0.0, axs = 0.0, ays = 0.0;
+        sum((int)M.cnt0[l], [&](int j) { return A.slots[g0 + j]; }, bx, by);
+        sum(n, [&](int j) {
+            if (!mat) return A.slots[at + j];
+            const uint32_t e = M.arena[at + j];
+            const int lc = (int)(e >> kEntryShift);
+            const int sl = A.slots[M.gstart[lc] + (int)(e & ((1u << kEntryShift) - 1))];
+            if (!kSerial) M.arena[at + j] = (uint32_t)sl | ((M.cflags[lc] & kCOwned) ? 0u : (uint32_t)kOwnBit);
+            return sl;
+        }, axs, ays);
+        const double ux = __ddiv_rn(__dsub_rn(bx, axs), (double)n);
+        const double uy = __ddiv_rn(__dsub_rn(by, ays), (double)n);
+        du2[l] = __dadd_rn(__dmul_rn(ux, ux), __dmul_rn(uy, uy));
+        if (wantDiag) {
+            const double ax = __ddiv_rn(axs, (double)n), ay = __ddiv_rn(ays, (double)n);
+            dgUx2 = __dadd_rn(dgUx2, __dmul_rn(ax, ax));
+            dgUy2 = __dadd_rn(dgUy2, __dmul_rn(ay, ay));
+            const double dpx = __dsub_rn(bx, axs), dpy = __dsub_rn(by, ays);
+            const double ex = __dmul_rn(dpx, dpx), ey = __dmul_rn(dpy, dpy);
+            if (ex > 0.0) { dgPx2 = __dadd_rn(dgPx2, ex); ++dgNPx; }
+            if (ey > 0.0) { dgPy2 = __dadd_rn(dgPy2, ey); ++dgNPy; }
+        }
+        bool doCorr = p.momCorr != 0;
+        if (doCorr && (f & kCSkip)) doCorr = false;
+        if (doCorr && (f & kCRecv) && !(f & kCBulkBulk)) doCorr = false;
+        doCorr = doCorr && (ux != 0.0 || uy != 0.0);
+        if (kSerial) {
+            // in place: every cell's sums must read the velocities of the zone's start
+            if (doCorr) A.duScratch[l] = make_double2(ux, uy);
+        } else if (doCorr && (mat || (f & kCOwned))) {
             for (int j0 = 0; j0 < n; j0 += 8) {
                 int sl[8];
                 double2 w[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    sl[u] = 0;
-                    if (j0 + u < n) {
-                        const uint32_t e = S.elem(l, j0 + u);
-                        sl[u] = A.slots[M.gstart[e >> kEntryShift] + (int)(e & ((1u << kEntryShift) - 1))];
-                    }
-                }
+                for (int u = 0; u < 8; ++u)
+                    sl[u] = (j0 + u >= n) ? kOwnBit : (mat ? (int)M.arena[at + j0 + u] : A.slots[at + j0 + u]);
 #pragma unroll
-                for (int u = 0; u < 8; ++u) w[u] = (j0 + u < n) ? zone_vin<kF32>(A, sl[u]) : make_double2(0.0, 0.0);
+                for (int u = 0; u < 8; ++u) w[u] = sl[u] >= 0 ? zone_vin<kF32>(A, sl[u]) : make_double2(0.0, 0.0);
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
-                    if (j0 + u < n) {
-                        axs = __dadd_rn(axs, w[u].x);
-                        ays = __dadd_rn(ays, w[u].y);
-                    }
-            }
-            const double ux = __ddiv_rn(__dsub_rn(bx, axs), (double)n);
-            const double uy = __ddiv_rn(__dsub_rn(by, ays), (double)n);
-            d2 = __dadd_rn(__dmul_rn(ux, ux), __dmul_rn(uy, uy));
-            if (wantDiag) {
-                const double ax = __ddiv_rn(axs, (double)n), ay = __ddiv_rn(ays, (double)n);
-                dgUx2 = __dadd_rn(dgUx2, __dmul_rn(ax, ax));
-                dgUy2 = __dadd_rn(dgUy2, __dmul_rn(ay, ay));
-                const double dpx = __dsub_rn(bx, axs), dpy = __dsub_rn(by, ays);
-                const double ex = __dmul_rn(dpx, dpx), ey = __dmul_rn(dpy, dpy);
-                if (ex > 0.0) { dgPx2 = __dadd_rn(dgPx2, ex); ++dgNPx; }
-                if (ey > 0.0) { dgPy2 = __dadd_rn(dgPy2, ey); ++dgNPy; }
-            }
-            bool doCorr = p.momCorr != 0;
-            if (doCorr && (f & kCSkip)) doCorr = false;
-            if (doCorr && (f & kCRecv) && !(f & kCBulkBulk)) doCorr = false;
-            if (kSerial) {
-                // in place: every cell's sums must read the velocities of the zone's start
-                A.duScratch[l] = (doCorr && (ux != 0.0 || uy != 0.0)) ? make_double2(ux, uy) : make_double2(0.0, 0.0);
-            } else if (doCorr && (ux != 0.0 || uy != 0.0)) {
-                for (int j = 0; j < n; ++j) {
-                    const uint32_t e = S.elem(l, j);
-                    const int lc = (int)(e >> kEntryShift);
-                    if (!(M.cflags[lc] & kCOwned)) continue;
-                    const int sl = A.slots[M.gstart[lc] + (int)(e & ((1u << kEntryShift) - 1))];
-                    const double2 w = zone_vin<kF32>(A, sl);
-                    zone_vout<kF32>(A, sl, make_double2(__dadd_rn(w.x, ux), __dadd_rn(w.y, uy)));
-                }
+                    if (sl[u] >= 0) zone_vout<kF32>(A, sl[u], make_double2(__dadd_rn(w[u].x, ux), __dadd_rn(w[u].y, uy)));
             }
         }
-        du2[l] = d2;
     }
     __syncwarp();
     if (wantDiag) {
@@ -1362,26 +1558,22 @@ __device__ __forceinline__ bool zone_finish(ZoneState<I, kF32>& S, const ZoneArg
         }
         __syncwarp();
     }
-    if (kSerial) serial_finish(S, A, p);
-    // zone stats[4], stats[5] (src/zone_pass.cpp:911-922): the sum of positive dU2 in
-    // ascending cell order and their maximum (zero entries change neither)
-    double acc = 0.0, mx = 0.0;
+    // zone stats[4], stats[5] (src/zone_pass.cpp:911-922): the sum of positive dU2 in ascending
+    // cell order (adding the zeros changes nothing) and the maximum of their roots (the root of the
+    // maximum: a correctly rounded root is monotone).
+    double acc = 0.0, top = 0.0;
     int cntDU = 0;
-    for (int b = 0; b < S.nl; b += kWarp) {
-        const int l = b + lane;
-        const double d2 = (l < S.nl) ? du2[l] : 0.0;
-        unsigned pos = __ballot_sync(0xffffffffu, d2 > 0.0);
-        while (pos) {
-            const int q = __ffs(pos) - 1;
-            pos &= pos - 1;
-            const double v = __shfl_sync(0xffffffffu, d2, q);
-            acc = __dadd_rn(acc, v);
-            mx = smax(mx, sqrt(v));
+    for (int l = 0; l < S.nl; ++l) {
+        const double d2 = du2[l];
+        if (d2 > 0.0) {
+            acc = __dadd_rn(acc, d2);
+            top = smax(top, d2);
             ++cntDU;
         }
     }
+    if (kSerial) serial_finish(S, A, p);
     if (lane == 0) {
-        A.zoneCorr[z] = make_double2((cntDU > 0) ? sqrt(__ddiv_rn(acc, (double)cntDU)) : 0.0, (cntDU > 0) ? mx : 0.0);
+        A.zoneCorr[z] = make_double2((cntDU > 0) ? sqrt(__ddiv_rn(acc, (double)cntDU)) : 0.0, sqrt(top));
         A.zoneMoved[z] = make_int2(S.movedDense, S.movedSparse);
     }
     return true;
