@@ -65,7 +65,6 @@ def build(force=False, verbose=False):
         "-ccbin", shutil.which("g++") or "g++",
         "-shared", "-I", os.path.join(ROOT, "include"), "-I", CSRC,
         "-o", OUT + ".tmp",
-        "--split-compile=0",
     ] + [os.path.join(CSRC, f) for f in SOURCES]
     if verbose:
         print(" ".join(cmd), file=sys.stderr)

@@ -232,9 +232,9 @@ __device__ __forceinline__ int srd_cell(double x, double y, double sx, double sy
 // mt19937_64(seed), which need seeded words 0, 1, 2, 156, 157 only. One thread.
 // stepCounter (graph replay): first begin the step on the device (step_begin), then draw its
 // shift from the device seed table
-__global__ void k_srd_shift(DevParams P, uint64_t seed, double* out, const uint64_t* seedDev,
-                            long long* stepCounter = nullptr, uint64_t* stepSeeds = nullptr) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__device__ __forceinline__ void srd_shift_block(const DevParams& P, uint64_t seed, double* out, const uint64_t* seedDev,
+                                                long long* stepCounter, uint64_t* stepSeeds) {
+    if (threadIdx.x != 0) return;
     if (stepCounter) step_begin(stepCounter, stepSeeds);
     if (seedDev) seed = seedDev[kSeedSrdShift];
     uint64_t w[kMtM + 2];
@@ -245,6 +245,9 @@ __global__ void k_srd_shift(DevParams P, uint64_t seed, double* out, const uint6
     const double a = __dmul_rn(-0.5, P.a0), b = __dmul_rn(0.5, P.a0);
     out[0] = __dadd_rn(__dmul_rn(canon(o0), __dsub_rn(b, a)), a);
     out[1] = __dadd_rn(__dmul_rn(canon(o1), __dsub_rn(b, a)), a);
+}
+__global__ void k_srd_shift(DevParams P, uint64_t seed, double* out) {
+    srd_shift_block(P, seed, out, nullptr, nullptr, nullptr);
 }
 
 // Streams (optional), replays the sweeps, and computes the cell ids the next phases need.

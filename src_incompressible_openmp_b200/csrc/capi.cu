@@ -98,6 +98,7 @@ struct mpcd_ctx {
     // positions in place and velocities out of place, so each pass flips xv and xflip together
     // (the positions stay in their buffer); a whole step leaves xflip as it found it.
     int xflip = 0;
+    int* redDone = nullptr;   // blocks finished of the reduction in progress (k_reduce_cols resets it)
     int* partFill = nullptr;  // kPartBuckets: bucket fill counts of the state's id-order output (state_io.cuh)
     int* cidStd = nullptr;
     int* cidSrd = nullptr;
@@ -113,6 +114,7 @@ struct mpcd_ctx {
     bool srdCellsValid = false;
     CellIndex idxStd, idxSrd;
     bool idxStdValid = false;
+    bool idxIota = false;  // the standard index's slots are the identity and not written yet (ensure_std_index)
     uint64_t* blockSums = nullptr;
     uint64_t* blockSumsWalls = nullptr;  // the walls' scan runs beside the index scans
     int blockSumsCap = 0;
@@ -143,7 +145,7 @@ struct mpcd_ctx {
     int64_t gkernels[8] = {};
     struct HostFlags {
         int xv, pp, xflip;
-        bool cidStdValid, srdCellsValid, idxStdValid, refValid;
+        bool cidStdValid, srdCellsValid, idxStdValid, idxIota, refValid;
     } gpost[8];
     cudaEvent_t signsReady[2] = {nullptr, nullptr};
     cudaEvent_t collDone = nullptr;
@@ -157,6 +159,12 @@ struct mpcd_ctx {
     // zones
     Layout lay[3];  // base, shifted, single_full
     uint64_t* seeds = nullptr;
+    // Where both passes' generator states stay small, a step makes them on their own stream at its
+    // start, off the chain of its phases (seedsEarly).
+    bool seedsEarly = false, seedsPending = false;
+    uint64_t* seedsShifted = nullptr;
+    cudaStream_t seedStream = nullptr;
+    cudaEvent_t stepBegun = nullptr, seedsDone = nullptr;
     int2* zoneMoved = nullptr;
     double2* zoneCorr = nullptr;
     int* overflow = nullptr;
@@ -362,6 +370,7 @@ int check_device(mpcd_ctx* c) {
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     if (c->side) CUDA_TRY(cudaStreamSynchronize(c->side));
     if (c->walls) CUDA_TRY(cudaStreamSynchronize(c->walls));
+    if (c->seedStream) CUDA_TRY(cudaStreamSynchronize(c->seedStream));
     CUDA_TRY(cudaMemcpy(c->hst, c->st, sizeof(DevStatus), cudaMemcpyDeviceToHost));
     if (c->hst->code != 0) {
         const int code = c->hst->code;
@@ -641,6 +650,7 @@ int build_index(mpcd_ctx* c, const int* cid, CellIndex& I, Prof* pf = nullptr, i
     if (!s) s = c->stream;
     if (!keys) keys = c->sortKeys;
     if (!sums) sums = c->blockSums;
+    if (&I == &c->idxStd) c->idxIota = false;
     if (c->n > 0) {
         k_histogram<<<blocks_for(c->n, kThreads * kIndexItems), kThreads, 0, s>>>(cid, c->n, I.count, I.pos);
         ++c->launches;
@@ -670,14 +680,25 @@ __global__ void k_set_step(long long* step, long long value) {
 }
 
 // the wall bitmaps and counters of a boundary sweep, cleared in one launch
-__global__ void k_walls_clear(BcWork W, int nwords) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void walls_clear_block(int blk, const BcWork& W, int nwords) {
+    const int i = blk * blockDim.x + threadIdx.x;
     if (i < nwords) {
         W.bitsX[i] = 0u;
         W.bitsY[i] = 0u;
     }
     if (i < 4) W.ints[i] = 0;
     if (i == 0) *W.nEvents = 0;
+}
+__global__ void k_walls_clear(BcWork W, int nwords) { walls_clear_block((int)blockIdx.x, W, nwords); }
+
+// The start of a step: block 0 begins it on the device (graph replay) and draws its SRD shift, the
+// others clear the wall bitmaps and counters.
+__global__ void k_step_head(DevParams P, uint64_t seed, const uint64_t* seedDev, long long* stepCounter,
+                            uint64_t* stepSeeds, BcWork W, int nwords) {
+    if (blockIdx.x == 0)
+        srd_shift_block(P, seed, W.srdShift, seedDev, stepCounter, stepSeeds);
+    else
+        walls_clear_block((int)blockIdx.x - 1, W, nwords);
 }
 
 // the particle state of slots [0, n) from S to T, in one launch
@@ -708,7 +729,15 @@ int ensure_std_index(mpcd_ctx* c, Prof* pf = nullptr) {
         CUDA_TRY(cudaStreamWaitEvent(c->stream, c->stdIdxDone, 0));
         c->stdIdxPending = false;
     }
-    if (c->idxStdValid) return MPCD_OK;
+    if (c->idxStdValid) {
+        // after a step the slots are in index order; most steps rebuild the index unread
+        if (c->idxIota) {
+            k_iota<<<blocks_for(c->n), kThreads, 0, c->stream>>>(c->idxStd.slots, c->n); ++c->launches;
+            CUDA_TRY(cudaGetLastError());
+            c->idxIota = false;
+        }
+        return MPCD_OK;
+    }
     if (!c->cidStdValid) {
         WITH_VIEW(c->xv, k_std_cells<<<blocks_for(c->n), kThreads, 0, c->stream>>>(c->P, S, c->cidStd));
         ++c->launches;
@@ -798,8 +827,8 @@ int reduce_cols(mpcd_ctx* c, const double* cols, int64_t rows, int K, unsigned m
     const int rowsPerBlock = 8192;
     const int nb = (int)std::max<int64_t>(1, (rows + rowsPerBlock - 1) / rowsPerBlock);
     if ((int64_t)nb * K > c->partialCap) return set_err(MPCD_ERR_CAPACITY, "reduction buffer too small");
-    k_reduce_partial<<<nb, kRedThreads, 0, c->stream>>>(cols, rows, K, maxMask, rowsPerBlock, c->partial); ++c->launches;
-    k_reduce_final<<<1, kRedThreads, 0, c->stream>>>(c->partial, nb, K, maxMask, out); ++c->launches;
+    k_reduce_cols<<<nb, kRedThreads, 0, c->stream>>>(cols, rows, K, maxMask, rowsPerBlock, c->partial, c->redDone, out);
+    ++c->launches;
     CUDA_TRY(cudaGetLastError());
     return MPCD_OK;
 }
@@ -810,7 +839,9 @@ int reduce_cols(mpcd_ctx* c, const double* cols, int64_t rows, int K, unsigned m
 int run_bc(mpcd_ctx* c, bool doStream, uint64_t seed, int* cidStd, int* cidSrd, bool wantInfo, Prof* pf = nullptr,
            bool overlap = false) {
     BcWork& W = c->W;
-    k_walls_clear<<<blocks_for(c->nwords), kThreads, 0, c->stream>>>(W, c->nwords); ++c->launches;
+    if (!doStream) {  // the step's k_step_head has cleared them
+        k_walls_clear<<<blocks_for(c->nwords), kThreads, 0, c->stream>>>(W, c->nwords); ++c->launches;
+    }
     if (wantInfo)
         WITH_VIEW(c->xv, k_stream_bc<true><<<c->bcBlocks, kThreads, 0, c->stream>>>(c->P, doStream ? 1 : 0, S, c->pidb[c->pp],
                                                                                    cidStd, cidSrd, W, c->st));
@@ -982,12 +1013,11 @@ int run_save_ref(mpcd_ctx* c, Prof* pf = nullptr, bool inStep = false) {
     if (rc) return rc;
     FieldsOut o{};
     o.N = c->refNi; o.Ux = c->refUx; o.Uy = c->refUy; o.Px = c->refPx; o.Py = c->refPy; o.T = c->refT;
-    o.rho = c->refRho; o.Pkin = c->refPkin; o.Pvir = c->refPvir; o.P = c->refP;
+    o.rho = c->refRho; o.Pkin = c->refPkin; o.Pvir = c->refPvir; o.P = c->refP;  // pdRaw: Pkin + Pvir is refP
     const int* skip = (inStep && c->learnedOn) ? c->lmode : nullptr;  // learned steps need no reference
     WITH_VIEW(c->xv, k_cell_fields<<<blocks_for(c->Nc), kThreads, 0, c->stream>>>(c->P, c->idxStd.start, c->idxStd.slots, S,
                                                                                   c->P.rhoTarget, o, skip));
     ++c->launches;
-    k_pdrive<<<blocks_for(c->Nc), kThreads, 0, c->stream>>>(c->P, c->refPkin, c->refPvir, c->pdRaw, skip); ++c->launches;
     k_pdrive_blend<<<blocks_for(c->Nc), kThreads, 0, c->stream>>>(c->P, c->pdRaw, c->mask, c->nMasked > 0, c->pdrive, skip);
     ++c->launches;
     k_eos<<<blocks_for(c->Nc), kThreads, 0, c->stream>>>(c->P, c->pdrive, c->eosX, c->eosY, skip); ++c->launches;
@@ -997,10 +1027,13 @@ int run_save_ref(mpcd_ctx* c, Prof* pf = nullptr, bool inStep = false) {
     return MPCD_OK;
 }
 
+constexpr int kSms = 148;
+constexpr int kZonesOneWave = 4 * kSms;  // zones that run one per block, all at once
+
 // The snapshot pass in three parts, so that a batch can run the middle one for all its
 // replicas in one launch: prep (index, seeds, output copies, launch order; fills c->zA),
 // the zone kernel, and finish (overflow zones, metrics, state flags).
-int zone_pass_prep(mpcd_ctx* c, int mode, uint64_t seedBase, Prof* pf = nullptr) {
+int zone_pass_prep(mpcd_ctx* c, int mode, uint64_t seedBase, Prof* pf = nullptr, bool inStep = false) {
     if (!c->cidStdValid) {
         WITH_VIEW(c->xv, k_std_cells<<<blocks_for(c->n), kThreads, 0, c->stream>>>(c->P, S, c->cidStd)); ++c->launches;
         c->cidStdValid = true;
@@ -1012,9 +1045,18 @@ int zone_pass_prep(mpcd_ctx* c, int mode, uint64_t seedBase, Prof* pf = nullptr)
     if (mode != MPCD_LAYOUT_SHIFTED && mode != MPCD_LAYOUT_SINGLE_FULL) mode = MPCD_LAYOUT_BASE;
     if (c->pc.zoneSingleFullDomainMode) mode = MPCD_LAYOUT_SINGLE_FULL;
     Layout& L = c->lay[mode];
-    k_zone_seeds<<<(L.nZones + kSeedZonesPerBlock - 1) / kSeedZonesPerBlock, kSeedZonesPerBlock * 2, 0, c->stream>>>(
-        seedBase, L.nZones, c->seeds, c->graphMode ? c->stepSeeds : nullptr, shiftedPass ? kSeedShifted : kSeedBase);
-    ++c->launches;
+    uint64_t* seeds = c->seeds;
+    if (inStep && c->seedsEarly) {  // made at the start of the step
+        if (shiftedPass) seeds = c->seedsShifted;
+        if (c->seedsPending) {
+            CUDA_TRY(cudaStreamWaitEvent(c->stream, c->seedsDone, 0));
+            c->seedsPending = false;
+        }
+    } else {
+        k_zone_seeds<<<(L.nZones + kSeedZonesPerBlock - 1) / kSeedZonesPerBlock, kSeedZonesPerBlock * 2, 0, c->stream>>>(
+            seedBase, L.nZones, seeds, c->graphMode ? c->stepSeeds : nullptr, shiftedPass ? kSeedShifted : kSeedBase);
+        ++c->launches;
+    }
     mark(c, pf, 7);
     // velocities out of place (output starts as a copy of the input; zones write what they
     // change), positions in place (the zone kernel never reads them)
@@ -1036,7 +1078,7 @@ int zone_pass_prep(mpcd_ctx* c, int mode, uint64_t seedBase, Prof* pf = nullptr)
     A.in32 = view32(c, xi);
     A.out32 = View32{c->offb[xi ^ c->xflip], c->cellb[xi ^ c->xflip], c->v32b[xo]};
     A.cid = c->cidStd;
-    A.seeds = c->seeds;
+    A.seeds = seeds;
     A.nZones = L.nZones;
     A.maxCells = c->zMaxCells;
     A.winCap = c->zWinCap;
@@ -1050,7 +1092,7 @@ int zone_pass_prep(mpcd_ctx* c, int mode, uint64_t seedBase, Prof* pf = nullptr)
     // heaviest zones first (by estimated dense-phase work) in the base pass; the shifted pass
     // runs after the base pass has evened the counts, its zones cost about the same, and the
     // two ordering kernels would cost more than the tail they save
-    if (mode == MPCD_LAYOUT_SHIFTED) {
+    if (mode == MPCD_LAYOUT_SHIFTED || L.nZones <= kZonesOneWave) {  // (all zones start at once)
         A.order = nullptr;
     } else {
         k_zone_cost<<<blocks_for(L.nZones), kThreads, 0, c->stream>>>(c->P, L.rects, c->idxStd.start, L.nZones,
@@ -1289,8 +1331,7 @@ int run_closure(mpcd_ctx* c, bool permute, bool wantRep, bool wantStats, Prof* p
         c->xv ^= 1;
         c->pp ^= 1;
         c->slotsSorted = true;
-        k_iota<<<blocks_for(c->n), kThreads, 0, c->stream>>>(c->idxStd.slots, c->n); ++c->launches;
-        CUDA_TRY(cudaGetLastError());
+        c->idxIota = true;
         mark(c, pf, 10);
         // the standard index stays valid (same cells, identity slots); per-slot cell ids and
         // SRD cells refer to the old layout
@@ -1327,13 +1368,15 @@ int mpcd_ctx_destroy(mpcd_ctx* c) {
     if (c->profP) cudaFree(c->profP);
     if (c->profN) cudaFree(c->profN);
     if (c->partFill) cudaFree(c->partFill);
+    if (c->redDone) cudaFree(c->redDone);
+    if (c->pdRaw == c->refP) c->pdRaw = nullptr;  // the slot forms' alias
     void* ptrs[] = {c->xb[0], c->xb[1], c->vb[0], c->vb[1], c->offb[0], c->offb[1], c->cellb[0], c->cellb[1],
                     c->v32b[0], c->v32b[1], c->pidb[0], c->pidb[1], c->cidStd, c->cidSrd, c->sortKeys, c->sortKeysSide,
                     c->idxStd.count, c->idxStd.start, c->idxStd.pos, c->idxStd.slots,
                     c->idxSrd.count, c->idxSrd.start, c->idxSrd.pos, c->idxSrd.slots,
                     c->blockSums, c->blockSumsWalls, c->W.bitsX, c->W.bitsY, c->W.wordCount, c->W.wordPrefix, c->W.events,
                     c->W.nEvents, c->W.normals, c->W.contrib, c->W.blockPartial, c->W.ints, c->W.srdShift,
-                    c->wallOut, c->signs, c->seeds, c->zoneMoved, c->zoneCorr, c->overflow, c->nOverflow, c->ovDone,
+                    c->wallOut, c->signs, c->seeds, c->seedsShifted, c->zoneMoved, c->zoneCorr, c->overflow, c->nOverflow, c->ovDone,
                     c->zoneCost, c->zoneHist, c->zoneOrder, c->dStep, c->stepSeeds,
                     c->slotsLive, c->liveCnt, c->liveStart, c->liveTop, c->duScratch, c->zkRect, c->zkDiag, c->zkOut,
                     c->lparams, c->lmode, c->lcount, c->lsums, c->duLX, c->duLY, c->duLSum, c->redFeat,
@@ -1350,9 +1393,10 @@ int mpcd_ctx_destroy(mpcd_ctx* c) {
         if (e) cudaEventDestroy(e);
     if (c->side) cudaStreamSynchronize(c->side);
     if (c->walls) cudaStreamSynchronize(c->walls);
+    if (c->seedStream) cudaStreamSynchronize(c->seedStream);
     for (cudaStream_t q : {c->up, c->down})
         if (q) cudaStreamSynchronize(q);
-    for (cudaEvent_t e : {c->signsReady[0], c->signsReady[1], c->collDone, c->bcDone, c->wallsDone, c->sideDone, c->stdIdxDone,
+    for (cudaEvent_t e : {c->signsReady[0], c->signsReady[1], c->collDone, c->bcDone, c->wallsDone, c->sideDone, c->stdIdxDone, c->stepBegun, c->seedsDone,
                           c->upDone[0], c->upDone[1], c->inFree[0], c->inFree[1], c->outReady[0], c->outReady[1],
                           c->downDone[0], c->downDone[1]})
         if (e) cudaEventDestroy(e);
@@ -1363,6 +1407,7 @@ int mpcd_ctx_destroy(mpcd_ctx* c) {
     for (auto& g : c->gexec)
         if (g) cudaGraphExecDestroy(g);
     if (c->side) cudaStreamDestroy(c->side);
+    if (c->seedStream) cudaStreamDestroy(c->seedStream);
     if (c->walls) cudaStreamDestroy(c->walls);
     if (c->signsBuf[0]) cudaFree(c->signsBuf[0]);
     if (c->signsBuf[1]) cudaFree(c->signsBuf[1]);
@@ -1404,7 +1449,8 @@ int mpcd_ctx_create_form(const mpcd_params_c* params, int device, int32_t form, 
     if (cudaSetDevice(device) != cudaSuccess) return fail(set_err(MPCD_ERR_CUDA, "cudaSetDevice failed"));
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(set_err(MPCD_ERR_CUDA, "stream"));
     const int n = c->n, Nc = c->Nc;
-    if ((rc = dalloc(&c->partFill, kPartBuckets))) return fail(rc);
+    if ((rc = dalloc(&c->partFill, kPartBuckets)) || (rc = dalloc(&c->redDone, 1))) return fail(rc);
+    if (cudaMemset(c->redDone, 0, sizeof(int)) != cudaSuccess) return fail(set_err(MPCD_ERR_CUDA, "reduction counter"));
     if (form == MPCD_FORM_FAST) {
         rc = fast_create(c, *params, device);
         if (rc) return fail(rc);
@@ -1491,6 +1537,20 @@ int mpcd_ctx_create_form(const mpcd_params_c* params, int device, int32_t form, 
         maxTY = std::max(maxTY, L.maxTY);
     }
     ALLOC(c->seeds, (size_t)maxZones * kMtN);
+    {
+        // 32 MB for both layouts: the states are read back from L2, which a step's other traffic
+        // leaves them in only while they are few (4096x1024: 2 x 105 MB, 0.45 ms slower early). At
+        // 25 zones the two launches in line cost 33 us of a 353 us step.
+        const int nz = c->lay[0].nZones + c->lay[1].nZones;
+        c->seedsEarly = (size_t)nz * kMtN * sizeof(uint64_t) <= (size_t)32 << 20;
+        if (c->seedsEarly) {
+            ALLOC(c->seedsShifted, (size_t)maxZones * kMtN);
+            if (cudaStreamCreateWithFlags(&c->seedStream, cudaStreamNonBlocking) != cudaSuccess ||
+                cudaEventCreateWithFlags(&c->stepBegun, cudaEventDisableTiming) != cudaSuccess ||
+                cudaEventCreateWithFlags(&c->seedsDone, cudaEventDisableTiming) != cudaSuccess)
+                return fail(set_err(MPCD_ERR_CUDA, "seed stream"));
+        }
+    }
     ALLOC(c->zoneMoved, (size_t)maxZones);
     ALLOC(c->zoneCorr, (size_t)maxZones);
     ALLOC(c->overflow, (size_t)maxZones);
@@ -1562,9 +1622,8 @@ int mpcd_ctx_create_form(const mpcd_params_c* params, int device, int32_t form, 
         // (0: one zone per block).
         c->zSyncWarps = 0;
         if (c->zMaxCells > 0) {
-            constexpr int kSms = 148;
             const int nz = std::max(B.nZones, S.nZones);
-            int W = nz <= 4 * kSms ? 0 : (nz <= 8 * kSms ? 4 : (nz <= 64 * kSms ? 8 : 16));
+            int W = nz <= kZonesOneWave ? 0 : (nz <= 8 * kSms ? 4 : (nz <= 64 * kSms ? 8 : 16));
             while (W > 0 && (size_t)W * c->zSmem > 200 * 1024) W = W > 4 ? W / 2 : 0;
             c->zSyncWarps = W;
         }
@@ -1600,8 +1659,9 @@ int mpcd_ctx_create_form(const mpcd_params_c* params, int device, int32_t form, 
     if (cudaMemcpy(c->mask, mask.data(), (size_t)Nc * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(set_err(MPCD_ERR_CUDA, "mask upload"));
     for (double** p : {&c->refPx, &c->refPy, &c->refUx, &c->refUy, &c->refT, &c->refRho, &c->refPkin, &c->refPvir,
-                       &c->refP, &c->pdRaw, &c->pdrive, &c->eosX, &c->eosY, &c->duRX, &c->duRY})
+                       &c->refP, &c->pdrive, &c->eosX, &c->eosY, &c->duRX, &c->duRY})
         ALLOC(*p, (size_t)Nc);
+    c->pdRaw = c->refP;
     ALLOC(c->refNi, (size_t)Nc);
     ALLOC(c->cols, (size_t)std::max<int64_t>((int64_t)Nc * kKickCols, 3LL * n));
     c->partialCap = (int)(((int64_t)std::max(Nc, n) + 8191) / 8192 + 1) * kRedMaxCols;
@@ -1749,7 +1809,7 @@ int mpcd_srd_shift_cells(mpcd_ctx* c, uint64_t seed, int32_t* cid_out) {
     if (!c) return set_err(MPCD_ERR_INVALID_ARG, "null context");
     if (c->f32 || c->fast) return set_err(MPCD_ERR_INVALID_ARG, "the FP32 precision and fast forms run the whole step only (mpcd_step*, state I/O, metrics)");
     CUDA_TRY(cudaSetDevice(c->device));
-    k_srd_shift<<<1, 1, 0, c->stream>>>(c->P, seed, c->W.srdShift, nullptr); ++c->launches;
+    k_srd_shift<<<1, 1, 0, c->stream>>>(c->P, seed, c->W.srdShift); ++c->launches;
     k_srd_cells<<<blocks_for(c->n), kThreads, 0, c->stream>>>(c->P, cur_x(c), c->W.srdShift, c->cidSrd); ++c->launches;
     CUDA_TRY(cudaGetLastError());
     c->srdCellsValid = true;
@@ -2249,9 +2309,27 @@ static int step_head(mpcd_ctx* c, int64_t step, bool metrics, Prof* pf) {
     const uint64_t s = (uint64_t)step;
     if (metrics) CUDA_TRY(cudaEventRecord(c->ev[0], c->stream));
     mark(c, pf, -1);
-    k_srd_shift<<<1, 1, 0, c->stream>>>(c->P, 130363ULL + 10007ULL * s, c->W.srdShift,
-                                        c->graphMode ? c->stepSeeds : nullptr, c->graphMode ? c->dStep : nullptr,
-                                        c->stepSeeds); ++c->launches;
+    k_step_head<<<1 + blocks_for(c->nwords), kThreads, 0, c->stream>>>(
+        c->P, 130363ULL + 10007ULL * s, c->graphMode ? c->stepSeeds : nullptr, c->graphMode ? c->dStep : nullptr,
+        c->stepSeeds, c->W, c->nwords);
+    ++c->launches;
+    CUDA_TRY(cudaGetLastError());
+    if (c->seedsEarly) {
+        // both passes' zone generators, beside the stream and the collision
+        const uint64_t base = 88172645463325252ULL + 10007ULL * s;
+        CUDA_TRY(cudaEventRecord(c->stepBegun, c->stream));
+        CUDA_TRY(cudaStreamWaitEvent(c->seedStream, c->stepBegun, 0));
+        const uint64_t* gs = c->graphMode ? c->stepSeeds : nullptr;
+        for (int pass = 0; pass < 2; ++pass) {
+            const int nz = c->lay[c->pc.zoneSingleFullDomainMode ? 2 : pass].nZones;
+            k_zone_seeds<<<(nz + kSeedZonesPerBlock - 1) / kSeedZonesPerBlock, kSeedZonesPerBlock * 2, 0, c->seedStream>>>(
+                base + (pass ? 4099ULL : 0ULL), nz, pass ? c->seedsShifted : c->seeds, gs, pass ? kSeedShifted : kSeedBase);
+            ++c->launches;
+        }
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaEventRecord(c->seedsDone, c->seedStream));
+        c->seedsPending = true;
+    }
     const bool overlap = pf == nullptr && c->walls;
     int rc = run_bc(c, true, 104729ULL + 10007ULL * s, c->cidStd, c->cidSrd, metrics, pf, overlap);
     if (rc) return rc;
@@ -2272,7 +2350,7 @@ static int step_head(mpcd_ctx* c, int64_t step, bool metrics, Prof* pf) {
     rc = run_save_ref(c, pf, true);
     if (rc) return rc;
     if (metrics) CUDA_TRY(cudaEventRecord(c->ev[1], c->stream));
-    return zone_pass_prep(c, MPCD_LAYOUT_BASE, 88172645463325252ULL + 10007ULL * s, pf);
+    return zone_pass_prep(c, MPCD_LAYOUT_BASE, 88172645463325252ULL + 10007ULL * s, pf, true);
 }
 
 static int step_mid_b(mpcd_ctx* c, int64_t step, bool metrics, Prof* pf) {
@@ -2286,7 +2364,7 @@ static int step_mid_b(mpcd_ctx* c, int64_t step, bool metrics, Prof* pf) {
         if (rc) return rc;
         CUDA_TRY(cudaEventRecord(c->ev[3], c->stream));
     }
-    return zone_pass_prep(c, MPCD_LAYOUT_SHIFTED, 88172645463325252ULL + 4099ULL + 10007ULL * s, pf);
+    return zone_pass_prep(c, MPCD_LAYOUT_SHIFTED, 88172645463325252ULL + 4099ULL + 10007ULL * s, pf, true);
 }
 
 static int step_mid(mpcd_ctx* c, int64_t step, bool metrics, Prof* pf) {
@@ -2318,6 +2396,8 @@ static int step_tail_b(mpcd_ctx* c, bool metrics, Prof* pf) {
         FieldsOut o{};
         o.Ux = c->fieldTmp;
         o.Uy = c->fieldTmp + c->Nc;
+        rc = ensure_std_index(c);
+        if (rc) return rc;
         WITH_VIEW(c->xv, k_cell_fields<<<blocks_for(c->Nc), kThreads, 0, c->stream>>>(c->P, c->idxStd.start, c->idxStd.slots,
                                                                                       S, c->P.rhoTarget, o));
         ++c->launches;
@@ -2373,7 +2453,7 @@ static int graph_step(mpcd_ctx* c, int64_t step) {
         }
         c->gkernels[key] = c->launches - l0;
         c->launches = l0;
-        c->gpost[key] = {c->xv, c->pp, c->xflip, c->cidStdValid, c->srdCellsValid, c->idxStdValid, c->refValid};
+        c->gpost[key] = {c->xv, c->pp, c->xflip, c->cidStdValid, c->srdCellsValid, c->idxStdValid, c->idxIota, c->refValid};
     } else {
         const auto& f = c->gpost[key];  // host-side state after the step, as step_once leaves it
         c->xv = f.xv;
@@ -2383,6 +2463,7 @@ static int graph_step(mpcd_ctx* c, int64_t step) {
         c->cidStdValid = f.cidStdValid;
         c->srdCellsValid = f.srdCellsValid;
         c->idxStdValid = f.idxStdValid;
+        c->idxIota = f.idxIota;
         c->refValid = f.refValid;
     }
     // the sign stream of this step may come from an eager step's prefetch on the side stream
@@ -2958,7 +3039,10 @@ static int batch_index(mpcd_batch* b) {
     }
     k_cell_rank_batch<<<b->rankBlocks, kRankThreads, 0, b->stream>>>(jobs, b->dOffsRank, n); ++c0->launches;
     CUDA_TRY(cudaGetLastError());
-    for (mpcd_ctx* c : b->members) c->idxStdValid = true;
+    for (mpcd_ctx* c : b->members) {
+        c->idxStdValid = true;
+        c->idxIota = false;
+    }
     return MPCD_OK;
 }
 
@@ -3031,7 +3115,7 @@ static int batch_graph_step(mpcd_batch* b, int64_t step) {
             mpcd_ctx* c = b->members[r];
             b->gkernels[key][r] = c->launches - l0[r];
             c->launches = l0[r];
-            b->gpost[key][r] = {c->xv, c->pp, c->xflip, c->cidStdValid, c->srdCellsValid, c->idxStdValid, c->refValid};
+            b->gpost[key][r] = {c->xv, c->pp, c->xflip, c->cidStdValid, c->srdCellsValid, c->idxStdValid, c->idxIota, c->refValid};
         }
     }
     for (int r = 0; r < n; ++r) {
@@ -3044,6 +3128,7 @@ static int batch_graph_step(mpcd_batch* b, int64_t step) {
         c->cidStdValid = f.cidStdValid;
         c->srdCellsValid = f.srdCellsValid;
         c->idxStdValid = f.idxStdValid;
+        c->idxIota = f.idxIota;
         c->refValid = f.refValid;
         CUDA_TRY(cudaStreamWaitEvent(b->stream, c->signsReady[step & 1], 0));
     }

@@ -1,7 +1,7 @@
 // Liquid closure (reference src/liquid_closure.cpp:329-444).
 //
 //   ref fields  : cell fields of the post-collision state (computed before the zone passes)
-//   k_pdrive    : pdriveRaw = Pkin + Pvir of ref, blended with the 5-point cross smoothing on
+//   k_pdrive_blend : pdriveRaw = Pkin + Pvir of ref (the fields' P), blended with the 5-point cross smoothing on
 //                 the static interzone mask (:401-419, local_cross_smooth :215-241)
 //   k_eos       : boundary-aware central gradient and the EOS kick (:243-295, :424-430)
 //   k_closure_cells : red-state momenta per cell, duRepair and the beta_opt terms (:343-360)
@@ -33,14 +33,6 @@ __device__ __forceinline__ double cross_smooth(const double* raw, int ix, int iy
 
 // skip (nullable): a device flag; when set, the step runs the learned closure and these
 // kernels of the plain one do nothing
-__global__ void k_pdrive(DevParams P, const double* __restrict__ pkin, const double* __restrict__ pvir, double* __restrict__ raw,
-                         const int* skip) {
-    if (skip && *skip) return;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= P.Nc) return;
-    raw[c] = __dadd_rn(pkin[c], pvir[c]);
-}
-
 __device__ __forceinline__ void pdrive_blend_block(int bx, const DevParams& P, const double* __restrict__ raw,
                                                    const int* __restrict__ mask, int anyMask, double* __restrict__ pdrive,
                                                    const int* skip) {
@@ -128,11 +120,12 @@ __global__ void k_closure_cells(DevParams P, const uint64_t* __restrict__ start,
 
 // ---------------------------------------------------------------- fixed-order reductions
 // K interleaved columns over n rows; kind bit k set -> max instead of sum for column k.
+// sh: shared memory, K rows or more.
 constexpr int kRedThreads = 256;
 constexpr int kRedMaxCols = 16;
 __device__ __forceinline__ void reduce_partial_block(int bx, const double* __restrict__ in, int64_t n, int K,
-                                                     unsigned maxMask, int rowsPerBlock, double* __restrict__ partial) {
-    __shared__ double sh[kRedMaxCols][kRedThreads];
+                                                     unsigned maxMask, int rowsPerBlock, double* partial,
+                                                     double (*sh)[kRedThreads]) {
     const int t = threadIdx.x;
     const int64_t r0 = (int64_t)bx * rowsPerBlock;
     const int64_t r1 = min((int64_t)n, r0 + rowsPerBlock);
@@ -154,20 +147,13 @@ __device__ __forceinline__ void reduce_partial_block(int bx, const double* __res
     if (t < K) partial[(size_t)bx * K + t] = sh[t][0];
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_reduce_partial(const double* __restrict__ in, int64_t n, int K,
-                                                                unsigned maxMask, int rowsPerBlock,
-                                                                double* __restrict__ partial) {
-    reduce_partial_block((int)blockIdx.x, in, n, K, maxMask, rowsPerBlock, partial);
-}
-
-__device__ __forceinline__ void reduce_final_block(const double* __restrict__ partial, int nb, int K, unsigned maxMask,
-                                                   double* __restrict__ out) {
-    __shared__ double sh[kRedMaxCols][kRedThreads];
+__device__ __forceinline__ void reduce_final_block(const double* partial, int nb, int K, unsigned maxMask,
+                                                   double* __restrict__ out, double (*sh)[kRedThreads]) {
     const int t = threadIdx.x;
     for (int k = 0; k < K; ++k) {
         double a = 0.0;
         for (int b = t; b < nb; b += kRedThreads) {
-            const double x = partial[(size_t)b * K + k];
+            const double x = __ldcg(partial + (size_t)b * K + k);  // may be another block's, of the same launch
             a = ((maxMask >> k) & 1u) ? smax(a, x) : __dadd_rn(a, x);
         }
         sh[k][t] = a;
@@ -182,9 +168,22 @@ __device__ __forceinline__ void reduce_final_block(const double* __restrict__ pa
     if (t < K) out[t] = sh[t][0];
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_reduce_final(const double* __restrict__ partial, int nb, int K,
-                                                              unsigned maxMask, double* __restrict__ out) {
-    reduce_final_block(partial, nb, K, maxMask, out);
+// Both stages in one launch: the last block to finish reduces the partials (in their fixed order,
+// so the result does not depend on which block that is) and resets *done.
+__global__ void __launch_bounds__(kRedThreads) k_reduce_cols(const double* __restrict__ in, int64_t n, int K,
+                                                             unsigned maxMask, int rowsPerBlock, double* partial,
+                                                             int* done, double* __restrict__ out) {
+    __shared__ double sh[kRedMaxCols][kRedThreads];
+    __shared__ int last;
+    reduce_partial_block((int)blockIdx.x, in, n, K, maxMask, rowsPerBlock, partial, sh);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (threadIdx.x == 0) *done = 0;
+    reduce_final_block(partial, (int)gridDim.x, K, maxMask, out, sh);
 }
 
 // beta_applied from num/den (src/liquid_closure.cpp:364-377)

@@ -174,19 +174,21 @@ __global__ void __launch_bounds__(256) k_fb_closure_cells(const FastClosureJob* 
 
 __global__ void __launch_bounds__(kRedThreads) k_fb_reduce_partial(const FastClosureJob* __restrict__ jobs,
                                                                    const int* __restrict__ offs, int n) {
+    __shared__ double sh[2][kRedThreads];
     __shared__ __align__(16) char sj[fb_bytes<FastClosureJob>()];
     const int r = fb_replica(offs, n, (int)blockIdx.x);
     if (r < 0) return;
     const FastClosureJob& J = fb_stage(jobs, r, sj);
-    reduce_partial_block((int)blockIdx.x - offs[r], J.cols, (int64_t)J.P.Nc, 2, 0u, kFastBatchRedRows, J.partial);
+    reduce_partial_block((int)blockIdx.x - offs[r], J.cols, (int64_t)J.P.Nc, 2, 0u, kFastBatchRedRows, J.partial, sh);
 }
 
 // one block per replica
 __global__ void __launch_bounds__(kRedThreads) k_fb_reduce_final(const FastClosureJob* __restrict__ jobs, int n) {
+    __shared__ double sh[2][kRedThreads];
     __shared__ __align__(16) char sj[fb_bytes<FastClosureJob>()];
     if ((int)blockIdx.x >= n) return;
     const FastClosureJob& J = fb_stage(jobs, (int)blockIdx.x, sj);
-    reduce_final_block(J.partial, J.nbRed, 2, 0u, J.numDen);
+    reduce_final_block(J.partial, J.nbRed, 2, 0u, J.numDen, sh);
 }
 
 __global__ void __launch_bounds__(256) k_fb_pdrive(const FastClosureJob* __restrict__ jobs, const int* __restrict__ offs,
