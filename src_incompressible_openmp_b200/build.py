@@ -13,7 +13,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libmpcd_b200.so")
 
-SOURCES = ["capi.cu", "io.cpp"]
+SOURCES = ["capi.cu", "zone.cu", "io.cpp"]
 DEPS = sorted(f for f in os.listdir(CSRC)
               if f.endswith((".cuh", ".inc", ".h")))
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -59,18 +59,29 @@ def build(force=False, verbose=False):
     if not force and not needs_build():
         build_driver(verbose)
         return OUT
-    cmd = [nvcc_path()] + ARCH + [
+    flags = ARCH + [
         "-O3", "-lineinfo", "-std=c++17", "-fmad=false",
         "-Xcompiler", "-fPIC,-ffp-contract=off",
         "-ccbin", shutil.which("g++") or "g++",
-        "-shared", "-I", os.path.join(ROOT, "include"), "-I", CSRC,
-        "-o", OUT + ".tmp",
-    ] + [os.path.join(CSRC, f) for f in SOURCES]
+        "-I", os.path.join(ROOT, "include"), "-I", CSRC,
+    ]
+    objs = [os.path.join(HERE, "build_" + os.path.splitext(f)[0] + ".o") for f in SOURCES]
+    cmds = [[nvcc_path()] + flags + ["-c", "-o", o, os.path.join(CSRC, f)] for f, o in zip(SOURCES, objs)]
+    link = [nvcc_path()] + ARCH + ["-ccbin", shutil.which("g++") or "g++", "-shared", "-o", OUT + ".tmp"] + objs
     if verbose:
-        print(" ".join(cmd), file=sys.stderr)
-    r = subprocess.run(cmd, capture_output=True, text=True)
+        for c in cmds + [link]:
+            print(" ".join(c), file=sys.stderr)
+    # one process per source, side by side
+    runs = [subprocess.Popen(c, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True) for c in cmds]
+    outs = [r.communicate()[0] for r in runs]
+    for r, o in zip(runs, outs):
+        if r.returncode != 0:
+            raise RuntimeError("nvcc failed:\n" + o)
+    r = subprocess.run(link, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("nvcc failed:\n" + r.stdout + r.stderr)
+    for o in objs:
+        os.remove(o)
     os.replace(OUT + ".tmp", OUT)
     build_driver(verbose)
     return OUT

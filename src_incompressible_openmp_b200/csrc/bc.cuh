@@ -253,9 +253,10 @@ __global__ void k_srd_shift(DevParams P, uint64_t seed, double* out) {
 // Streams (optional), replays the sweeps, and computes the cell ids the next phases need.
 // S: slot-ordered state. cidStd: cell on the standard grid; cidSrd (optional): SRD cell.
 template <bool kInfo, class V>
-__global__ void k_stream_bc(DevParams P, int doStream, V S, const int* __restrict__ pid, int* __restrict__ cidStd,
-                            int* __restrict__ cidSrd, BcWork W, DevStatus* st) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void stream_bc_block(int blk, const DevParams& P, int doStream, const V& S,
+                                                const int* __restrict__ pid, int* __restrict__ cidStd,
+                                                int* __restrict__ cidSrd, const BcWork& W, DevStatus* st) {
+    const int s = blk * blockDim.x + threadIdx.x;
     double acc[kWallDoubles];
     for (int k = 0; k < kWallDoubles; ++k) acc[k] = 0.0;
     int nhit[4] = {0, 0, 0, 0};
@@ -321,23 +322,31 @@ __global__ void k_stream_bc(DevParams P, int doStream, V S, const int* __restric
     if (threadIdx.x < kWallDoubles) {
         double a = 0.0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) a = __dadd_rn(a, sh[threadIdx.x][w]);
-        W.blockPartial[blockIdx.x * kWallDoubles + threadIdx.x] = a;
+        W.blockPartial[blk * kWallDoubles + threadIdx.x] = a;
     }
 }
+template <bool kInfo, class V>
+__global__ void k_stream_bc(DevParams P, int doStream, V S, const int* __restrict__ pid, int* __restrict__ cidStd,
+                            int* __restrict__ cidSrd, BcWork W, DevStatus* st) {
+    stream_bc_block<kInfo>((int)blockIdx.x, P, doStream, S, pid, cidStd, cidSrd, W, st);
+}
 
+__device__ __forceinline__ void word_counts_block(int blk, const uint32_t* __restrict__ bx, const uint32_t* __restrict__ by,
+                                                  int nwords, uint64_t* __restrict__ cnt) {
+    const int w = blk * blockDim.x + threadIdx.x;
+    if (w < nwords) cnt[w] = (uint64_t)(__popc(bx[w]) + __popc(by[w]));
+}
 __global__ void k_word_counts(const uint32_t* __restrict__ bx, const uint32_t* __restrict__ by, int nwords,
                               uint64_t* __restrict__ cnt) {
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w < nwords) cnt[w] = (uint64_t)(__popc(bx[w]) + __popc(by[w]));
+    word_counts_block((int)blockIdx.x, bx, by, nwords, cnt);
 }
 
 // One block of 320 threads generates pairs 0 .. nPairs-1 of normal_distribution(0,1) on
 // mt19937_64(seed): attempt a uses draws 2a, 2a+1; accepted attempts become pairs in
 // order; pair p = (y*mult, x*mult) = (first deviate, cached second deviate).
 constexpr int kNormThreads = 320;
-__global__ void __launch_bounds__(kNormThreads) k_wall_normals(uint64_t seed, const uint64_t* __restrict__ totalPairs,
-                                                             int cap, double* __restrict__ normals, DevStatus* st,
-                                                             const uint64_t* seedDev) {
+__device__ __forceinline__ void wall_normals_block(uint64_t seed, const uint64_t* __restrict__ totalPairs, int cap,
+                                                   double* __restrict__ normals, DevStatus* st, const uint64_t* seedDev) {
     if (seedDev) seed = seedDev[kSeedBc];
     __shared__ uint64_t mt[kMtN];
     __shared__ uint64_t scanSh[32];
@@ -393,12 +402,17 @@ __global__ void __launch_bounds__(kNormThreads) k_wall_normals(uint64_t seed, co
         __syncthreads();
     }
 }
+__global__ void __launch_bounds__(kNormThreads) k_wall_normals(uint64_t seed, const uint64_t* __restrict__ totalPairs,
+                                                             int cap, double* __restrict__ normals, DevStatus* st,
+                                                             const uint64_t* seedDev) {
+    wall_normals_block(seed, totalPairs, cap, normals, st, seedDev);
+}
 
 // Thermal particles: replay with their pairs; write the final velocity and the WallInfo
 // contribution at the slot of their first pair.
 template <class V>
-__global__ void k_wall_apply(DevParams P, V S, BcWork W, DevStatus* st) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void wall_apply_block(int blk, const DevParams& P, const V& S, const BcWork& W, DevStatus* st) {
+    const int e = blk * blockDim.x + threadIdx.x;
     const int ne = min(*W.nEvents, W.eventCap);
     if (e >= ne) return;
     const WallEvent ev = W.events[e];
@@ -425,6 +439,10 @@ __global__ void k_wall_apply(DevParams P, V S, BcWork W, DevStatus* st) {
     }
     for (int k = 0; k < 4; ++k)
         if (nhit[k]) atomicAdd(&W.ints[k], nhit[k]);
+}
+template <class V>
+__global__ void k_wall_apply(DevParams P, V S, BcWork W, DevStatus* st) {
+    wall_apply_block((int)blockIdx.x, P, S, W, st);
 }
 
 // WallInfo doubles: block partials of k_stream_bc then per-pair contributions, in order.

@@ -27,6 +27,7 @@
 #include "closure.cuh"
 #include "common.cuh"
 #include "fast.cuh"
+#include "f64_batch.cuh"
 #include "fast_batch.cuh"
 #include "learned.cuh"
 #include "sort.cuh"
@@ -159,11 +160,10 @@ struct mpcd_ctx {
     // zones
     Layout lay[3];  // base, shifted, single_full
     uint64_t* seeds = nullptr;
-    // Where both passes' generator states stay small, a step makes them on their own stream at its
+    // Where both passes' generator states stay small, a step makes them on the side stream at its
     // start, off the chain of its phases (seedsEarly).
     bool seedsEarly = false, seedsPending = false;
     uint64_t* seedsShifted = nullptr;
-    cudaStream_t seedStream = nullptr;
     cudaEvent_t stepBegun = nullptr, seedsDone = nullptr;
     int2* zoneMoved = nullptr;
     double2* zoneCorr = nullptr;
@@ -370,7 +370,6 @@ int check_device(mpcd_ctx* c) {
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     if (c->side) CUDA_TRY(cudaStreamSynchronize(c->side));
     if (c->walls) CUDA_TRY(cudaStreamSynchronize(c->walls));
-    if (c->seedStream) CUDA_TRY(cudaStreamSynchronize(c->seedStream));
     CUDA_TRY(cudaMemcpy(c->hst, c->st, sizeof(DevStatus), cudaMemcpyDeviceToHost));
     if (c->hst->code != 0) {
         const int code = c->hst->code;
@@ -488,24 +487,28 @@ std::vector<int> interzone_mask(const mpcd_params_c& p, const Layout& base, cons
             }
         return b;
     };
+    // a square window: along y, then along x
     auto dilate = [&](const std::vector<int>& in) {
         const int w = p.smoothPdriveInterzoneWidthCells;
         if (w <= 0) return in;
-        std::vector<int> out((size_t)p.Nc, 0);
-        for (int ix = 0; ix < p.Nx; ++ix)
-            for (int iy = 0; iy < p.Ny; ++iy) {
-                bool on = false;
-                for (int dx = -w; dx <= w && !on; ++dx)
-                    for (int dy = -w; dy <= w; ++dy) {
-                        int jx = ix + dx, jy = iy + dy;
-                        if (px) jx = ((jx % p.Nx) + p.Nx) % p.Nx;
-                        else if (jx < 0 || jx >= p.Nx) continue;
-                        if (py) jy = ((jy % p.Ny) + p.Ny) % p.Ny;
-                        else if (jy < 0 || jy >= p.Ny) continue;
-                        if (in[(size_t)jy + (size_t)p.Ny * jx]) { on = true; break; }
-                    }
-                out[(size_t)iy + (size_t)p.Ny * ix] = on;
+        auto reach = [w](int i, int N, bool per, auto on) {
+            for (int d = -w; d <= w; ++d) {
+                int j = i + d;
+                if (per) j = ((j % N) + N) % N;
+                else if (j < 0 || j >= N) continue;
+                if (on(j)) return 1;
             }
+            return 0;
+        };
+        std::vector<int> mid((size_t)p.Nc, 0), out((size_t)p.Nc, 0);
+        for (int ix = 0; ix < p.Nx; ++ix)
+            for (int iy = 0; iy < p.Ny; ++iy)
+                mid[(size_t)iy + (size_t)p.Ny * ix] =
+                    reach(iy, p.Ny, py, [&](int j) { return in[(size_t)j + (size_t)p.Ny * ix] != 0; });
+        for (int ix = 0; ix < p.Nx; ++ix)
+            for (int iy = 0; iy < p.Ny; ++iy)
+                out[(size_t)iy + (size_t)p.Ny * ix] =
+                    reach(ix, p.Nx, px, [&](int j) { return mid[(size_t)iy + (size_t)p.Ny * j] != 0; });
         return out;
     };
     mask = dilate(boundary(base.howner));
@@ -1008,12 +1011,17 @@ int run_collide(mpcd_ctx* c, uint64_t seed, Prof* pf = nullptr, int64_t step = -
 
 // reference fields of the current state + pdrive + EOS kick (depend on the reference only);
 // inStep: called from the step, where a learned step (device mode flag) skips them
-int run_save_ref(mpcd_ctx* c, Prof* pf = nullptr, bool inStep = false) {
-    int rc = ensure_std_index(c, pf);
-    if (rc) return rc;
+FieldsOut ref_fields(const mpcd_ctx* c) {
     FieldsOut o{};
     o.N = c->refNi; o.Ux = c->refUx; o.Uy = c->refUy; o.Px = c->refPx; o.Py = c->refPy; o.T = c->refT;
     o.rho = c->refRho; o.Pkin = c->refPkin; o.Pvir = c->refPvir; o.P = c->refP;  // pdRaw: Pkin + Pvir is refP
+    return o;
+}
+
+int run_save_ref(mpcd_ctx* c, Prof* pf = nullptr, bool inStep = false) {
+    int rc = ensure_std_index(c, pf);
+    if (rc) return rc;
+    const FieldsOut o = ref_fields(c);
     const int* skip = (inStep && c->learnedOn) ? c->lmode : nullptr;  // learned steps need no reference
     WITH_VIEW(c->xv, k_cell_fields<<<blocks_for(c->Nc), kThreads, 0, c->stream>>>(c->P, c->idxStd.start, c->idxStd.slots, S,
                                                                                   c->P.rhoTarget, o, skip));
@@ -1025,6 +1033,38 @@ int run_save_ref(mpcd_ctx* c, Prof* pf = nullptr, bool inStep = false) {
     mark(c, pf, 6);
     c->refValid = true;
     return MPCD_OK;
+}
+
+// The zone kernel's arguments for layout `mode` on view xi of the state, positions addressed with
+// xflip (launch order: by id)
+ZoneArgs zone_args(const mpcd_ctx* c, int mode, int xi, int xflip, const uint64_t* seeds) {
+    const Layout& L = c->lay[mode];
+    const int xo = xi ^ 1;
+    ZoneArgs A{};
+    A.P = c->P;
+    A.rects = L.rects;
+    A.owner = L.owner;
+    A.start = c->idxStd.start;
+    A.slots = c->idxStd.slots;
+    A.vin = c->vb[xi];
+    A.xout = c->xb[xi ^ xflip];
+    A.vout = c->vb[xo];
+    A.f32 = c->f32 ? 1 : 0;
+    A.in32 = View32{c->offb[xi ^ xflip], c->cellb[xi ^ xflip], c->v32b[xi]};
+    A.out32 = View32{c->offb[xi ^ xflip], c->cellb[xi ^ xflip], c->v32b[xo]};
+    A.cid = c->cidStd;
+    A.seeds = seeds;
+    A.nZones = L.nZones;
+    A.maxCells = c->zMaxCells;
+    A.winCap = c->zWinCap;
+    A.arenaCap = c->zArenaCap;
+    A.nsmCap = c->zNsmCap;
+    A.overflow = c->overflow;
+    A.nOverflow = c->nOverflow;
+    A.zoneMoved = c->zoneMoved;
+    A.zoneCorr = c->zoneCorr;
+    A.st = c->st;
+    return A;
 }
 
 constexpr int kSms = 148;
@@ -1065,30 +1105,7 @@ int zone_pass_prep(mpcd_ctx* c, int mode, uint64_t seedBase, Prof* pf = nullptr,
         WITH_VIEWS(xi, xo, k_copy_vel<<<blocks_for(c->n), kThreads, 0, c->stream>>>(S, T, c->n));
         ++c->launches;
     }
-    ZoneArgs A{};
-    A.P = c->P;
-    A.rects = L.rects;
-    A.owner = L.owner;
-    A.start = c->idxStd.start;
-    A.slots = c->idxStd.slots;
-    A.vin = c->vb[xi];
-    A.xout = cur_x(c);
-    A.vout = c->vb[xo];
-    A.f32 = c->f32 ? 1 : 0;
-    A.in32 = view32(c, xi);
-    A.out32 = View32{c->offb[xi ^ c->xflip], c->cellb[xi ^ c->xflip], c->v32b[xo]};
-    A.cid = c->cidStd;
-    A.seeds = seeds;
-    A.nZones = L.nZones;
-    A.maxCells = c->zMaxCells;
-    A.winCap = c->zWinCap;
-    A.arenaCap = c->zArenaCap;
-    A.nsmCap = c->zNsmCap;
-    A.overflow = c->overflow;
-    A.nOverflow = c->nOverflow;
-    A.zoneMoved = c->zoneMoved;
-    A.zoneCorr = c->zoneCorr;
-    A.st = c->st;
+    ZoneArgs A = zone_args(c, mode, xi, c->xflip, seeds);
     // heaviest zones first (by estimated dense-phase work) in the base pass; the shifted pass
     // runs after the base pass has evened the counts, its zones cost about the same, and the
     // two ordering kernels would cost more than the tail they save
@@ -1132,9 +1149,9 @@ int zone_pass_kernel(mpcd_ctx* c) {
 // the overflow kernel's job for the pass in progress (its arguments with the global-memory
 // working set's capacities); the pass metrics (a serial sum over the zones) only if wanted:
 // the phase API and the metrics step of mpcd_step report them, plain steps do not
-OverflowJob overflow_job(const mpcd_ctx* c, bool metrics) {
+OverflowJob overflow_job(const mpcd_ctx* c, const ZoneArgs& A, double* metricsOut) {
     OverflowJob J{};
-    J.A = c->zA;
+    J.A = A;
     J.A.order = nullptr;
     J.A.maxCells = c->ovMaxCells;
     J.A.winCap = c->ovWinCap;
@@ -1143,8 +1160,11 @@ OverflowJob overflow_job(const mpcd_ctx* c, bool metrics) {
     J.gmem = c->ovMem;
     J.perBlock = c->ovPerBlock;
     J.blocksDone = c->ovDone;
-    J.metricsOut = metrics ? c->passOut + (c->zMode == MPCD_LAYOUT_SHIFTED ? 4 : 0) : nullptr;
+    J.metricsOut = metricsOut;
     return J;
+}
+OverflowJob overflow_job(const mpcd_ctx* c, bool metrics) {
+    return overflow_job(c, c->zA, metrics ? c->passOut + (c->zMode == MPCD_LAYOUT_SHIFTED ? 4 : 0) : nullptr);
 }
 
 // host-side state after a pass: velocities in the other buffer, positions in place
@@ -1393,7 +1413,6 @@ int mpcd_ctx_destroy(mpcd_ctx* c) {
         if (e) cudaEventDestroy(e);
     if (c->side) cudaStreamSynchronize(c->side);
     if (c->walls) cudaStreamSynchronize(c->walls);
-    if (c->seedStream) cudaStreamSynchronize(c->seedStream);
     for (cudaStream_t q : {c->up, c->down})
         if (q) cudaStreamSynchronize(q);
     for (cudaEvent_t e : {c->signsReady[0], c->signsReady[1], c->collDone, c->bcDone, c->wallsDone, c->sideDone, c->stdIdxDone, c->stepBegun, c->seedsDone,
@@ -1407,7 +1426,6 @@ int mpcd_ctx_destroy(mpcd_ctx* c) {
     for (auto& g : c->gexec)
         if (g) cudaGraphExecDestroy(g);
     if (c->side) cudaStreamDestroy(c->side);
-    if (c->seedStream) cudaStreamDestroy(c->seedStream);
     if (c->walls) cudaStreamDestroy(c->walls);
     if (c->signsBuf[0]) cudaFree(c->signsBuf[0]);
     if (c->signsBuf[1]) cudaFree(c->signsBuf[1]);
@@ -1545,10 +1563,9 @@ int mpcd_ctx_create_form(const mpcd_params_c* params, int device, int32_t form, 
         c->seedsEarly = (size_t)nz * kMtN * sizeof(uint64_t) <= (size_t)32 << 20;
         if (c->seedsEarly) {
             ALLOC(c->seedsShifted, (size_t)maxZones * kMtN);
-            if (cudaStreamCreateWithFlags(&c->seedStream, cudaStreamNonBlocking) != cudaSuccess ||
-                cudaEventCreateWithFlags(&c->stepBegun, cudaEventDisableTiming) != cudaSuccess ||
+            if (cudaEventCreateWithFlags(&c->stepBegun, cudaEventDisableTiming) != cudaSuccess ||
                 cudaEventCreateWithFlags(&c->seedsDone, cudaEventDisableTiming) != cudaSuccess)
-                return fail(set_err(MPCD_ERR_CUDA, "seed stream"));
+                return fail(set_err(MPCD_ERR_CUDA, "seed events"));
         }
     }
     ALLOC(c->zoneMoved, (size_t)maxZones);
@@ -2318,16 +2335,16 @@ static int step_head(mpcd_ctx* c, int64_t step, bool metrics, Prof* pf) {
         // both passes' zone generators, beside the stream and the collision
         const uint64_t base = 88172645463325252ULL + 10007ULL * s;
         CUDA_TRY(cudaEventRecord(c->stepBegun, c->stream));
-        CUDA_TRY(cudaStreamWaitEvent(c->seedStream, c->stepBegun, 0));
+        CUDA_TRY(cudaStreamWaitEvent(c->side, c->stepBegun, 0));
         const uint64_t* gs = c->graphMode ? c->stepSeeds : nullptr;
         for (int pass = 0; pass < 2; ++pass) {
             const int nz = c->lay[c->pc.zoneSingleFullDomainMode ? 2 : pass].nZones;
-            k_zone_seeds<<<(nz + kSeedZonesPerBlock - 1) / kSeedZonesPerBlock, kSeedZonesPerBlock * 2, 0, c->seedStream>>>(
+            k_zone_seeds<<<(nz + kSeedZonesPerBlock - 1) / kSeedZonesPerBlock, kSeedZonesPerBlock * 2, 0, c->side>>>(
                 base + (pass ? 4099ULL : 0ULL), nz, pass ? c->seedsShifted : c->seeds, gs, pass ? kSeedShifted : kSeedBase);
             ++c->launches;
         }
         CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaEventRecord(c->seedsDone, c->seedStream));
+        CUDA_TRY(cudaEventRecord(c->seedsDone, c->side));
         c->seedsPending = true;
     }
     const bool overlap = pf == nullptr && c->walls;
@@ -2944,9 +2961,15 @@ extern "C" int mpcd_cell_fields_static(const mpcd_params_c* params, const double
 // advance together. Each step is issued for every replica before the next step, each replica
 // on its own streams and from its own step graph, so their kernels run side by side on the GPU.
 struct FastBatch;
+struct F64Batch;
 struct mpcd_batch {
     int device = 0;
     FastBatch* fast = nullptr;  // fast-form replicas: one launch per phase (fast_batch.inc)
+    F64Batch* f64 = nullptr;    // plain replicas, one launch per phase (f64_batch.inc), made at the first step it takes
+    // the members' status codes gathered by one kernel (batch_status)
+    DevStatus** dStatus = nullptr;
+    int* dCodes = nullptr;
+    int* hCodes = nullptr;
     std::vector<mpcd_ctx*> members;
     cudaStream_t stream = nullptr;  // timing and the fork/join of the members' streams
     cudaEvent_t start = nullptr, stop = nullptr, fork = nullptr;
@@ -2977,12 +3000,31 @@ struct mpcd_batch {
     int histBlocks = 0, rankBlocks = 0;
 };
 
-#include "fast_batch.inc"
-
-__global__ void k_set_steps(long long** steps, int n, long long value) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) *steps[i] = value;
+// The device status of every member after a batched call, whose work is all on the batch stream: the
+// codes in one copy, then check_device of the first member that raised one.
+static int batch_status(mpcd_batch* b) {
+    const int n = (int)b->members.size();
+    if (!b->dStatus) {
+        std::vector<DevStatus*> st;
+        for (mpcd_ctx* c : b->members) st.push_back(c->st);
+        CUDA_TRY(cudaMallocHost((void**)&b->hCodes, sizeof(int) * (size_t)n));
+        int rc = dalloc(&b->dCodes, (size_t)n);
+        if (!rc) rc = dalloc(&b->dStatus, (size_t)n);
+        if (rc) return rc;
+        CUDA_TRY(cudaMemcpy(b->dStatus, st.data(), sizeof(DevStatus*) * (size_t)n, cudaMemcpyHostToDevice));
+    }
+    k_gather_status<<<(n + 255) / 256, 256, 0, b->stream>>>(b->dStatus, n, b->dCodes);
+    ++b->members[0]->launches;
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cudaMemcpyAsync(b->hCodes, b->dCodes, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, b->stream));
+    CUDA_TRY(cudaStreamSynchronize(b->stream));
+    for (int r = 0; r < n; ++r)
+        if (b->hCodes[r]) return check_device(b->members[(size_t)r]);
+    return MPCD_OK;
 }
+
+#include "fast_batch.inc"
+#include "f64_batch.inc"
 
 // the zone kernels of pass `pass` (0 base, 1 shifted) of every replica in one launch; each
 // replica's zone_pass_prep has filled its zA
@@ -3172,6 +3214,10 @@ int mpcd_batch_destroy(mpcd_batch* b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     fast_batch_free(b->fast);
+    f64_batch_free(b->f64);
+    if (b->dStatus) cudaFree(b->dStatus);
+    if (b->dCodes) cudaFree(b->dCodes);
+    if (b->hCodes) cudaFreeHost(b->hCodes);
     for (auto& g : b->gexec)
         if (g) cudaGraphExecDestroy(g);
     if (b->hArgs) cudaFreeHost(b->hArgs);
@@ -3338,6 +3384,20 @@ int mpcd_batch_step(mpcd_batch* b, int64_t step0, int64_t nsteps, double* device
         if (!c->pc.useIncompressibleRedistribution || !c->pc.useZoneRedistribution || !c->pc.useLiquidClosure)
             return set_err(MPCD_ERR_INVALID_ARG, "the benchmark step needs useIncompressibleRedistribution, useZoneRedistribution and useLiquidClosure");
     CUDA_TRY(cudaSetDevice(b->device));
+    bool together = true;
+    for (mpcd_ctx* c : b->members) together = together && f64_batch_takes(c);
+    if (together) {
+        for (mpcd_ctx* c : b->members) CUDA_TRY(cudaStreamSynchronize(c->stream));
+        CUDA_TRY(cudaEventRecord(b->start, b->stream));
+        const int rc = f64_batch_steps(b, step0, nsteps);
+        if (rc) return rc;
+        CUDA_TRY(cudaEventRecord(b->stop, b->stream));
+        CUDA_TRY(cudaEventSynchronize(b->stop));
+        float ms = 0.f;
+        CUDA_TRY(cudaEventElapsedTime(&ms, b->start, b->stop));
+        if (device_seconds) *device_seconds = ms * 1e-3;
+        return batch_status(b);
+    }
     CUDA_TRY(cudaEventRecord(b->start, b->stream));
     for (mpcd_ctx* c : b->members) CUDA_TRY(cudaStreamWaitEvent(c->stream, b->start, 0));
     for (int64_t k = 1; k <= nsteps; ++k) {

@@ -11,8 +11,8 @@ namespace mpcd_dev {
 // U(0,1) < 0.5 (theta = -alpha). One block generates `count` draws, one twist at a time.
 constexpr int kSignThreads = 320;
 // seedDev (graph replay): the next step's seed and output buffer (sign, sign1 by its parity)
-__global__ void __launch_bounds__(kSignThreads) k_srd_signs(uint64_t seed, int count, uint8_t* __restrict__ sign,
-                                                           const uint64_t* seedDev, uint8_t* sign1) {
+__device__ __forceinline__ void srd_signs_block(uint64_t seed, int count, uint8_t* sign, const uint64_t* seedDev,
+                                                uint8_t* sign1) {
     if (seedDev) {
         seed = seedDev[kSeedSignsNext];
         if (seedDev[kSeedNextParity]) sign = sign1;
@@ -44,6 +44,10 @@ __global__ void __launch_bounds__(kSignThreads) k_srd_signs(uint64_t seed, int c
         if (t < kMtN && base + t < count) sign[base + t] = (canon(mt_temper(mt[t])) < 0.5) ? 1 : 0;
         __syncthreads();
     }
+}
+__global__ void __launch_bounds__(kSignThreads) k_srd_signs(uint64_t seed, int count, uint8_t* __restrict__ sign,
+                                                           const uint64_t* seedDev, uint8_t* sign1) {
+    srd_signs_block(seed, count, sign, seedDev, sign1);
 }
 
 // srd_collision_step (src/srd_collision.cpp:47-124) on one SRD cell whose m velocities are
@@ -110,17 +114,16 @@ constexpr int kCollideShapes = 7;
 constexpr CollideShape kCollideShape[kCollideShapes] = {{32, 128}, {64, 256}, {128, 256}, {256, 512},
                                                         {16, 128}, {32, 256},  {16, 64}};
 
-template <class V, int kCollideCells, int kCollideThreads>
-__global__ void __launch_bounds__(kCollideThreads) k_srd_collide(DevParams P, const uint64_t* __restrict__ start,
-                                                                 const int* __restrict__ slots,
-                                                                 const uint8_t* __restrict__ sign, int signCount,
-                                                                 V S, DevStatus* st,
-                                                                 const uint64_t* seedDev,
-                                                                 const uint8_t* __restrict__ sign1, int tileCap) {
-    extern __shared__ __align__(16) double2 tv[];
+// smem: tileCap velocities, then as many slots
+template <class V, int kCollideCells>
+__device__ __forceinline__ void srd_collide_block(int blk, char* smem, const DevParams& P,
+                                                  const uint64_t* __restrict__ start, const int* __restrict__ slots,
+                                                  const uint8_t* sign, int signCount, const V& S, DevStatus* st,
+                                                  const uint64_t* seedDev, const uint8_t* sign1, int tileCap) {
+    double2* tv = reinterpret_cast<double2*>(smem);
     int* ts = reinterpret_cast<int*>(tv + tileCap);
     if (seedDev && seedDev[kSeedParity]) sign = sign1;
-    const int c0 = blockIdx.x * kCollideCells;
+    const int c0 = blk * kCollideCells;
     const int nc = min(kCollideCells, P.Nc - c0);
     const int A = (int)(uint32_t)start[c0], B = (int)(uint32_t)start[c0 + nc];
     const int t = threadIdx.x;
@@ -152,6 +155,18 @@ __global__ void __launch_bounds__(kCollideThreads) k_srd_collide(DevParams P, co
     for (int i = t; i < B - A; i += blockDim.x) S.set_vel(ts[i], tv[i]);
 }
 
+template <class V, int kCollideCells, int kCollideThreads>
+__global__ void __launch_bounds__(kCollideThreads) k_srd_collide(DevParams P, const uint64_t* __restrict__ start,
+                                                                 const int* __restrict__ slots,
+                                                                 const uint8_t* __restrict__ sign, int signCount,
+                                                                 V S, DevStatus* st,
+                                                                 const uint64_t* seedDev,
+                                                                 const uint8_t* __restrict__ sign1, int tileCap) {
+    extern __shared__ __align__(16) char smem[];
+    srd_collide_block<V, kCollideCells>((int)blockIdx.x, smem, P, start, slots, sign, signCount, S, st, seedDev, sign1,
+                                        tileCap);
+}
+
 struct FieldsOut {
     int* N;
     double *Ux, *Uy, *Px, *Py, *T, *rho, *Pkin, *Pvir, *P, *rhoTarget;
@@ -159,10 +174,10 @@ struct FieldsOut {
 
 // compute_cell_fields (src/common_grid.cpp:32-100), one cell per thread.
 template <class V>
-__global__ void k_cell_fields(DevParams Pm, const uint64_t* __restrict__ start, const int* __restrict__ slots, V S,
-                              double rhoTarget, FieldsOut o, const int* skip = nullptr) {
-    if (skip && *skip) return;  // a learned-closure step needs no reference fields
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void cell_fields_block(int blk, const DevParams& Pm, const uint64_t* __restrict__ start,
+                                                  const int* __restrict__ slots, const V& S, double rhoTarget,
+                                                  const FieldsOut& o) {
+    const int c = blk * blockDim.x + threadIdx.x;
     if (c >= Pm.Nc) return;
     const int a = (int)(uint32_t)start[c], b = (int)(uint32_t)start[c + 1];
     const int m = b - a;
@@ -202,6 +217,12 @@ __global__ void k_cell_fields(DevParams Pm, const uint64_t* __restrict__ start, 
     if (o.Pvir) o.Pvir[c] = pv;
     if (o.P) o.P[c] = __dadd_rn(pk, pv);
     if (o.rhoTarget) o.rhoTarget[c] = rhoTarget;
+}
+template <class V>
+__global__ void k_cell_fields(DevParams Pm, const uint64_t* __restrict__ start, const int* __restrict__ slots, V S,
+                              double rhoTarget, FieldsOut o, const int* skip = nullptr) {
+    if (skip && *skip) return;  // a learned-closure step needs no reference fields
+    cell_fields_block((int)blockIdx.x, Pm, start, slots, S, rhoTarget, o);
 }
 
 }  // namespace mpcd_dev

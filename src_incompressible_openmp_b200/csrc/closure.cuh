@@ -53,10 +53,9 @@ __global__ void k_pdrive_blend(DevParams P, const double* __restrict__ raw, cons
     pdrive_blend_block((int)blockIdx.x, P, raw, mask, anyMask, pdrive, skip);
 }
 
-__global__ void k_eos(DevParams P, const double* __restrict__ pd, double* __restrict__ eosX, double* __restrict__ eosY,
-                      const int* skip) {
-    if (skip && *skip) return;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void eos_block(int blk, const DevParams& P, const double* __restrict__ pd,
+                                          double* __restrict__ eosX, double* __restrict__ eosY) {
+    const int c = blk * blockDim.x + threadIdx.x;
     if (c >= P.Nc) return;
     const int ix = c / P.Ny, iy = c - ix * P.Ny;
     double gx, gy;
@@ -72,6 +71,11 @@ __global__ void k_eos(DevParams P, const double* __restrict__ pd, double* __rest
     eosX[c] = __dmul_rn(__dmul_rn(k, gx), P.betaEOS);
     eosY[c] = __dmul_rn(__dmul_rn(k, gy), P.betaEOS);
 }
+__global__ void k_eos(DevParams P, const double* __restrict__ pd, double* __restrict__ eosX, double* __restrict__ eosY,
+                      const int* skip) {
+    if (skip && *skip) return;
+    eos_block((int)blockIdx.x, P, pd, eosX, eosY);
+}
 
 // Per cell of the red (post-redistribution) state: momenta in particle-id order, velocity,
 // duRepair = (P_ref - P_red) / gamma and the beta_opt terms. cols: 2 doubles per cell
@@ -82,12 +86,14 @@ struct RedFields {
     float4* feat;  // (N/gamma - 1, Ux, Uy, N) as FP32: the learned closure's stencil input
 };
 template <class V>
-__global__ void k_closure_cells(DevParams P, const uint64_t* __restrict__ start, const int* __restrict__ slots, V S,
-                                const double* __restrict__ refPx,
-                                const double* __restrict__ refPy, const double* __restrict__ refUx,
-                                const double* __restrict__ refUy, RedFields red, double* __restrict__ duRX,
-                                double* __restrict__ duRY, double* __restrict__ cols, int* __restrict__ cellOf) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void closure_cells_block(int blk, const DevParams& P, const uint64_t* __restrict__ start,
+                                                    const int* __restrict__ slots, const V& S,
+                                                    const double* __restrict__ refPx, const double* __restrict__ refPy,
+                                                    const double* __restrict__ refUx, const double* __restrict__ refUy,
+                                                    const RedFields& red, double* __restrict__ duRX,
+                                                    double* __restrict__ duRY, double* __restrict__ cols,
+                                                    int* __restrict__ cellOf) {
+    const int c = blk * blockDim.x + threadIdx.x;
     if (c >= P.Nc) return;
     const int a = (int)(uint32_t)start[c], b = (int)(uint32_t)start[c + 1];
     const int m = b - a;
@@ -116,6 +122,14 @@ __global__ void k_closure_cells(DevParams P, const uint64_t* __restrict__ start,
     if (red.Ux) red.Ux[c] = ux;
     if (red.Uy) red.Uy[c] = uy;
     if (red.feat) red.feat[c] = make_float4((float)__dsub_rn(__ddiv_rn((double)m, P.gamma), 1.0), (float)ux, (float)uy, (float)m);
+}
+template <class V>
+__global__ void k_closure_cells(DevParams P, const uint64_t* __restrict__ start, const int* __restrict__ slots, V S,
+                                const double* __restrict__ refPx,
+                                const double* __restrict__ refPy, const double* __restrict__ refUx,
+                                const double* __restrict__ refUy, RedFields red, double* __restrict__ duRX,
+                                double* __restrict__ duRY, double* __restrict__ cols, int* __restrict__ cellOf) {
+    closure_cells_block((int)blockIdx.x, P, start, slots, S, refPx, refPy, refUx, refUy, red, duRX, duRY, cols, cellOf);
 }
 
 // ---------------------------------------------------------------- fixed-order reductions
@@ -257,13 +271,14 @@ __global__ void k_kick(DevParams P, const uint64_t* __restrict__ start, const in
 // particle mean) are computed once per block.
 constexpr int kKickItems = 2;
 template <class V>
-__global__ void k_kick_flat(DevParams P, int n, const int* __restrict__ cellOf, const int* __restrict__ slots,
-                            const double* __restrict__ numden, const double* __restrict__ duRX,
-                            const double* __restrict__ duRY, const double* __restrict__ eosX,
-                            const double* __restrict__ eosY, V S, const int* __restrict__ pid, V T,
-                            int* __restrict__ pido, const int* learned,
-                            const double* __restrict__ duLX, const double* __restrict__ duLY,
-                            const long long* __restrict__ duLSum) {
+__device__ __forceinline__ void kick_flat_block(int blk, const DevParams& P, int n, const int* __restrict__ cellOf,
+                                                const int* __restrict__ slots, const double* __restrict__ numden,
+                                                const double* __restrict__ duRX, const double* __restrict__ duRY,
+                                                const double* __restrict__ eosX, const double* __restrict__ eosY,
+                                                const V& S, const int* __restrict__ pid, const V& T,
+                                                int* __restrict__ pido, const int* learned,
+                                                const double* __restrict__ duLX, const double* __restrict__ duLY,
+                                                const long long* __restrict__ duLSum) {
     __shared__ double fac[2];  // beta, or the learned kick's particle mean (x, y)
     __shared__ int lrn;
     if (threadIdx.x == 0) {
@@ -278,7 +293,7 @@ __global__ void k_kick_flat(DevParams P, int n, const int* __restrict__ cellOf, 
         }
     }
     __syncthreads();
-    const int j0 = blockIdx.x * (blockDim.x * kKickItems) + threadIdx.x;
+    const int j0 = blk * (blockDim.x * kKickItems) + threadIdx.x;
     int c[kKickItems], s[kKickItems];
 #pragma unroll
     for (int k = 0; k < kKickItems; ++k) {
@@ -309,6 +324,17 @@ __global__ void k_kick_flat(DevParams P, int n, const int* __restrict__ cellOf, 
         T.copy_pos(j, S, s[k]);
         pido[j] = q[k];
     }
+}
+template <class V>
+__global__ void k_kick_flat(DevParams P, int n, const int* __restrict__ cellOf, const int* __restrict__ slots,
+                            const double* __restrict__ numden, const double* __restrict__ duRX,
+                            const double* __restrict__ duRY, const double* __restrict__ eosX,
+                            const double* __restrict__ eosY, V S, const int* __restrict__ pid, V T,
+                            int* __restrict__ pido, const int* learned,
+                            const double* __restrict__ duLX, const double* __restrict__ duLY,
+                            const long long* __restrict__ duLSum) {
+    kick_flat_block((int)blockIdx.x, P, n, cellOf, slots, numden, duRX, duRY, eosX, eosY, S, pid, T, pido, learned, duLX,
+                    duLY, duLSum);
 }
 
 // identity cell index after a permuting kick: slots[j] = j

@@ -226,7 +226,7 @@ __host__ __device__ __forceinline__ uint64_t mt_seed_next(uint64_t prev, int i) 
 
 // Out-of-place twist of a 312-word state A into B by one warp (A is left intact). Not
 // inlined: it is reached from every RNG call site and would otherwise bloat the zone kernel.
-__device__ __noinline__ void mt_twist_warp(const uint64_t* A, uint64_t* B, int lane) {
+static __device__ __noinline__ void mt_twist_warp(const uint64_t* A, uint64_t* B, int lane) {
     for (int i = lane; i < kMtN - kMtM; i += kWarp) B[i] = A[i + kMtM] ^ mt_mix(A[i], A[i + 1]);
     __syncwarp();
     for (int i = kMtN - kMtM + lane; i < kMtN - 1; i += kWarp) B[i] = B[i - (kMtN - kMtM)] ^ mt_mix(A[i], A[i + 1]);
@@ -305,7 +305,7 @@ struct WarpMt {
 };
 
 // log_cr as an out-of-line device function (shared by all call sites)
-__device__ __noinline__ double log_cr_dev(double x) { return mpcd_dd::log_cr(x); }
+static __device__ __noinline__ double log_cr_dev(double x) { return mpcd_dd::log_cr(x); }
 
 // normal_distribution<double>(0, 1): Marsaglia polar method with one cached deviate
 struct PolarNormal {
