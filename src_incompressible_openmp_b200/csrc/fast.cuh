@@ -62,7 +62,12 @@ struct FastStep {
 
 struct FastParams {
     int K;
-    int zoneWY;                  // unused padding for alignment
+    // the threshold maps as integers, [map 0 low, 1 high][cell occupied at the map build]: for a count
+    // n, n < map <=> n < cut, n > map <=> n > flo, floor(map - n) = flo - n for n <= map, and the
+    // deficit in units of 2^-12, rint((map - n) 4096), is map12 - 4096 n
+    int cut[2][2], flo[2][2];
+    int reserved;
+    long long map12[2][2];
     double fqx, fqy;             // body force * dt in grid units (fractional)
     float dtqx, dtqy;            // cell units moved per grid unit of velocity in one step
     double sigmaQ, UtopQ, UbottomQ;  // wall temperature and wall speeds in grid units
@@ -1014,6 +1019,12 @@ struct FastZone {
     int x0, x1, y0, y1, TX, TY, nl, WY;
     uint64_t zseed;
     uint32_t op;        // operation counter (salts the draws)
+    // this lane's range-2 neighbour (lanes 0 .. 23, kFastNb): its step, the offsets of its local cell
+    // and window index, and its place among the three of its angular bin by (chebyshev, distance^2),
+    // which are distinct there; direct: no wrapped neighbour of a zone cell lies in the zone
+    int ndx, ndy, nOff, nOffW;
+    uint32_t nOrd;
+    bool direct;
     int nrec;
     bool failed;        // out of records: remaining moves skipped
     int movedDense, movedSparse;
@@ -1021,8 +1032,28 @@ struct FastZone {
     __device__ __forceinline__ int cnt(int l) const { return M.win[M.wi[l]]; }
     __device__ __forceinline__ void add_cnt(int l, int d) { M.win[M.wi[l]] += (short)d; }
     __device__ __forceinline__ int gcell(int l) const { return (y0 + M.cy[l]) + A->P.Ny * (x0 + M.cx[l]); }
-    __device__ __forceinline__ double low_map(bool bulk) const { return bulk ? A->P.lowThrBulk : A->F.lowMapEmpty; }
-    __device__ __forceinline__ double high_map(bool bulk) const { return bulk ? A->P.highThr : A->F.highMapEmpty; }
+    __device__ __forceinline__ int bulk_d(int l) const { return (M.flg[l] & kZBulkD) ? 1 : 0; }
+    __device__ __forceinline__ void init_neighbours() {
+        const DevParams& P = A->P;
+        direct = (!P.perx || TX < P.Nx - 2) && (!P.pery || TY < P.Ny - 2);
+        ndx = ndy = nOff = nOffW = 0;
+        nOrd = 0;
+        if (lane < 24) {
+            ndx = kFastNb[lane][0];
+            ndy = kFastNb[lane][1];
+            nOff = ndx * TY + ndy;
+            nOffW = ndx * WY + ndy;
+            auto far = [](int dx, int dy) { return (max(abs(dx), abs(dy)) << 4) | (dx * dx + dy * dy); };
+            const int b = lane / 3 * 3, me = far(ndx, ndy);
+            for (int k = b; k < b + 3; ++k) nOrd += far(kFastNb[k][0], kFastNb[k][1]) < me;
+        }
+    }
+    // ceil(n - high map), in integers where the FP64 subtraction is exact
+    __device__ __forceinline__ int excess(int n, int cls) const {
+        const int h = A->F.flo[1][cls];
+        if (n <= 2 * h) return max(0, n - h);
+        return max(0, (int)ceil((double)n - (cls ? A->P.highThr : A->F.highMapEmpty)));
+    }
 
     // the zone cell at local (lx + dx, ly + dy), wrapping periodic axes; -1 outside the domain
     // or outside the zone
@@ -1042,20 +1073,36 @@ struct FastZone {
         return ((fmix64(zseed ^ ((uint64_t)salt << 32) ^ (uint64_t)pid) >> 41) << 31) | (uint64_t)(pid & 0x7fffffffu);
     }
 
+    // the particle ids of cell l's slots lane, lane + 32, .. (those the cell has)
+    struct Pids {
+        int p0, p1, p2, p3;
+    };
+    __device__ __forceinline__ Pids load_pids(int l) const {
+        const int* p = A->b.pid + (size_t)gcell(l) * A->F.K + lane;
+        const int n0 = M.n0[l];
+        Pids q{0, 0, 0, 0};
+        if (lane < n0) q.p0 = p[0];
+        if (n0 > 32) {
+            if (lane + 32 < n0) q.p1 = p[32];
+            if (lane + 64 < n0) q.p2 = p[64];
+            if (lane + 96 < n0) q.p3 = p[96];
+        }
+        return q;
+    }
+
     // The candidates of source cell l, one key per original not yet removed: slot j in lane
     // j % 32, register j / 32. A candidate is (key << 10) | (record flag << 9) | index: keys of at
     // most 54 bits whose low 31 bits are the particle id, original slots below 128 and records
     // below 512.
-    __device__ __forceinline__ void load_candidates(int l, bool dense, uint32_t salt, Cands& cand) const {
-        const FastBins& B = A->b;
-        const size_t ib = (size_t)gcell(l) * A->F.K;
+    __device__ __forceinline__ void load_candidates(int l, bool dense, uint32_t salt, const Pids& q, Cands& cand) const {
         const int n0 = M.n0[l];
+        const int pid[4] = {q.p0, q.p1, q.p2, q.p3};
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int j = lane + 32 * r;
             unsigned long long v = ~0ULL;
             if (j < n0 && !(M.rm[4 * l + r] & (1u << lane)))
-                v = (member_key(dense, salt, (uint32_t)B.pid[ib + j], -1) << 10) | (unsigned long long)j;
+                v = (member_key(dense, salt, (uint32_t)pid[r], -1) << 10) | (unsigned long long)j;
             cand.set(r, v);
         }
     }
@@ -1067,7 +1114,7 @@ struct FastZone {
     // random (the sparse phase shuffles the donor's list) from candidates keyed afresh.
     __device__ __forceinline__ void move_members(int l, int t, int nt, bool dense, Cands& cand) {
         const uint32_t salt = ++op;
-        if (!dense) load_candidates(l, false, salt, cand);
+        if (!dense) load_candidates(l, false, salt, load_pids(l), cand);
         for (int k = 0; k < nt; ++k) {
             if (failed) return;
             unsigned long long best = cand.lowest();
@@ -1112,21 +1159,32 @@ struct FastZone {
 
     // spread_particles_from_dense_source_round_robin (src/zone_pass.cpp:527-589) over the
     // targets ranked as rank_dense_targets_unified does (:436-490); map: 0 low, 1 high.
-    // Returns the particles moved; the receivers go to rcv[*nr ...].
+    // Returns the particles moved; the receivers go to rcv[*nr ...]. Comparisons and deficits are
+    // integers (FastParams::cut, flo, map12); the rank key's last part, a random tie-break, is never
+    // reached, since the neighbours of a bin differ in (chebyshev, distance^2).
     __device__ __forceinline__ int spread(int l, int needOut, int mapKind, int* rcv, int* nr, Cands& cand) {
-        // lane k < 24: the k-th neighbour of the bin-grouped offset table
-        const int k = lane;
-        int t = -1, ddx = 0, ddy = 0;
-        double map = 0.0;
+        const FastParams& F = A->F;
+        int t = -1, tc = 0, def = 0;
         bool adm = false;
-        if (k < 24) {
-            ddx = kFastNb[k][0];
-            ddy = kFastNb[k][1];
-            t = neighbour(l, ddx, ddy);
+        uint32_t key = 0xFFFFFFFFu;
+        if (lane < 24) {
+            if (direct) {
+                const bool in = (unsigned)(M.cx[l] + ndx) < (unsigned)TX && (unsigned)(M.cy[l] + ndy) < (unsigned)TY;
+                t = in ? l + nOff : -1;
+                tc = in ? M.win[M.wi[l] + nOffW] : 0;
+            } else {
+                t = neighbour(l, ndx, ndy);
+                tc = t >= 0 ? cnt(t) : 0;
+            }
             if (t >= 0) {
-                const bool bulk = M.flg[t] & kZBulkD;
-                map = mapKind ? high_map(bulk) : low_map(bulk);
-                adm = (double)cnt(t) < map;
+                const int cls = bulk_d(t);
+                adm = tc < F.cut[mapKind][cls];
+                if (adm) {
+                    // sort key (-deficit, cnt, chebyshev, distance^2); inward weight is 0 here
+                    const long long dq = min(F.map12[mapKind][cls] - 4096LL * tc, 0xFFFFFLL);
+                    key = ((0xFFFFFu - (uint32_t)dq) << 12) | ((uint32_t)min(tc, 255) << 4) | nOrd;
+                    def = max(0, F.flo[mapKind][cls] - tc);
+                }
             }
         }
         const unsigned admMask = __ballot_sync(0xffffffffu, adm);
@@ -1134,42 +1192,19 @@ struct FastZone {
         if (T == 0) return 0;
         const uint32_t salt = ++op;
         const int startBin = (int)(fmix64(zseed ^ ((uint64_t)salt << 12) ^ 0x42494EULL) >> 61);
-        // sort key (-deficit, cnt, chebyshev, distance^2, random); inward weight is 0 here
-        unsigned long long key = ~0ULL;
-        if (adm) {
-            const double deficit = fmax(0.0, map - (double)cnt(t));
-            const unsigned long long dq = (unsigned long long)min(llrint(deficit * 4096.0), (long long)0xFFFFF);
-            const int cheb = max(abs(ddx), abs(ddy)), d2 = ddx * ddx + ddy * ddy;
-            key = ((0xFFFFFULL - dq) << 44) | ((unsigned long long)min(cnt(t), 255) << 36) |
-                  ((unsigned long long)cheb << 34) | ((unsigned long long)d2 << 30) |
-                  (fmix64(zseed ^ ((uint64_t)salt << 8) ^ (uint64_t)k) & 0x3FFFFFFFULL);
-        }
         // rank inside the bin: the two other lanes of the bin
-        const int b = k / 3, base = 3 * b;
-        const unsigned long long ka = __shfl_sync(0xffffffffu, key, base + ((k - base + 1) % 3));
-        const unsigned long long kb = __shfl_sync(0xffffffffu, key, base + ((k - base + 2) % 3));
+        const int b = lane / 3, base = 3 * b;
+        const uint32_t ka = __shfl_sync(0xffffffffu, key, base + ((lane - base + 1) % 3));
+        const uint32_t kb = __shfl_sync(0xffffffffu, key, base + ((lane - base + 2) % 3));
         const int rank = (ka < key) + (kb < key);
         const int pos = rank * 8 + ((b - startBin + 8) & 7);
-        const unsigned posMask = __reduce_or_sync(0xffffffffu, adm ? (1u << pos) : 0u);
-        const int ord = __popc(posMask & ((1u << pos) - 1u));
-        if (adm) M.tgt[ord] = t;
-        __syncwarp();
-        // per ordered target (lane o < T): its current integer deficit
-        int def = 0;
-        double mapO = 0.0;
-        int tO = -1;
-        if (lane < T) {
-            tO = M.tgt[lane];
-            const bool bulk = M.flg[tO] & kZBulkD;
-            mapO = mapKind ? high_map(bulk) : low_map(bulk);
-            def = max(0, (int)floor(mapO - (double)cnt(tO)));
-        }
+        const unsigned below = (1u << (pos & 31)) - 1u;
         int avail = cnt(l);
         // With at most as many particles to move as targets with a deficit, the round-robin
         // quota stays 1: the first needOut of those targets (in order) take one particle each,
         // the i-th the i-th member in list order, drawn as the general loop below draws them
         // (its i-th call's salt, first draw). Done in one step when the source holds no records.
-        const unsigned defMask = __ballot_sync(0xffffffffu, lane < T && def > 0);
+        const unsigned defMask = __reduce_or_sync(0xffffffffu, adm && def > 0 ? (1u << pos) : 0u);
         if (needOut > 0 && needOut <= __popc(defMask) && needOut <= avail && M.nrecv[l] == 0 && !failed &&
             nrec + needOut <= A->recCap) {
             unsigned long long mine = ~0ULL;
@@ -1179,23 +1214,22 @@ struct FastZone {
                 cand.take(j, lane);
                 if (lane == i) mine = best;
             }
-            const int drank = __popc(defMask & lanemask_lt());
-            __syncwarp();
-            if (lane < T && def > 0 && drank < needOut) M.tgt[drank] = tO;
+            const int drank = __popc(defMask & below);
+            if (adm && def > 0 && drank < needOut) M.tgt[drank] = t;
             __syncwarp();
             if (lane < needOut) {
-                const int t = M.tgt[lane];
+                const int tt = M.tgt[lane];
                 const int j = (int)(mine & 511ULL);
-                const uint32_t salt = op + 1 + (uint32_t)lane;
+                const uint32_t msalt = op + 1 + (uint32_t)lane;
                 const int rec = nrec + lane;
                 M.recPid[rec] = (int)((mine >> 10) & 0x7fffffffULL);
                 M.recSrc[rec] = (uint16_t)((l << 7) | j);
-                M.recCur[rec] = (uint8_t)t;
-                M.recDraw[rec] = salt << 8;
-                M.nrecv[t] += 1;
-                add_cnt(t, 1);
+                M.recCur[rec] = (uint8_t)tt;
+                M.recDraw[rec] = msalt << 8;
+                M.nrecv[tt] += 1;
+                add_cnt(tt, 1);
                 atomicOr(&M.rm[4 * l + (j >> 5)], 1u << (j & 31));
-                rcv[*nr + lane] = t;
+                rcv[*nr + lane] = tt;
             }
             if (lane == 0) add_cnt(l, -needOut);
             op += (uint32_t)needOut;
@@ -1203,6 +1237,17 @@ struct FastZone {
             *nr += needOut;
             __syncwarp();
             return needOut;
+        }
+        // the general loop: per ordered target (lane o < T) its current integer deficit
+        const unsigned posMask = __reduce_or_sync(0xffffffffu, adm ? (1u << pos) : 0u);
+        if (adm) M.tgt[__popc(posMask & below)] = t;
+        __syncwarp();
+        int tO = -1, floO = 0;
+        def = 0;
+        if (lane < T) {
+            tO = M.tgt[lane];
+            floO = F.flo[mapKind][bulk_d(tO)];
+            def = max(0, floO - cnt(tO));
         }
         int moved = 0;
         unsigned got = 0;
@@ -1222,7 +1267,7 @@ struct FastZone {
                     add_cnt(tt, nt);
                 }
                 __syncwarp();
-                if (lane == kk) def = max(0, (int)floor(mapO - (double)cnt(tO)));
+                if (lane == kk) def = max(0, floO - cnt(tO));
                 got |= 1u << kk;
                 avail -= nt;
                 needOut -= nt;
@@ -1259,20 +1304,18 @@ struct FastZone {
 
     // redistribute_dense_cell_at_range_zone_local (src/zone_pass.cpp:591-634) and the mask
     // update of the dense loop (:745-750)
-    __device__ void dense_cell(int l) {
-        const bool bulk = M.flg[l] & kZBulkD;
-        const double hi = high_map(bulk);
+    __device__ void dense_cell(int l, const Pids& pids) {
+        const int cls = bulk_d(l);
         const int nc = cnt(l);
-        if (nc <= 0 || (double)nc <= hi) return;
-        const int needOut = max(0, (int)ceil((double)nc - hi));
+        if (nc <= 0 || nc <= A->F.flo[1][cls]) return;
         int nr = 0;
         int moved = 0;
         Cands cand;
-        load_candidates(l, true, 0, cand);
+        load_candidates(l, true, 0, pids, cand);
         // the low map first, then the high map for what is left (one call site: code size)
 #pragma unroll 1
         for (int phase = 0; phase < 2; ++phase) {
-            const int out = phase == 0 ? needOut : max(0, (int)ceil((double)cnt(l) - hi));
+            const int out = phase == 0 ? excess(nc, cls) : excess(cnt(l), cls);
             if (out <= 0 || failed) continue;
             moved += spread(l, out, phase, M.tgt2, &nr, cand);
         }
@@ -1661,6 +1704,7 @@ __device__ __forceinline__ void fast_zone_block(int bx, const FastZoneArgs& A, c
         Z.op = 0;
         Z.nrec = 0;
         Z.movedDense = Z.movedSparse = 0;
+        Z.init_neighbours();
         if (Z.nl > A.maxCells || (Z.TX + 4) * Z.WY > A.winCap || (Z.TX + 2) * (Z.TY + 2) > A.nsmCap) {
             if (lane == 0) raise_error(A.st, kErrZoneCapacity, z);
             ok = false;
@@ -1704,12 +1748,17 @@ __device__ __forceinline__ void fast_zone_block(int bx, const FastZoneArgs& A, c
             }
             __syncwarp();
             const int D = Z.order_cells([&](int i) -> uint32_t {
-                const bool bulk = M.flg[i] & kZBulkD;
-                if ((double)Z.cnt(i) > Z.high_map(bulk))
+                if (Z.cnt(i) > A.F.flo[1][Z.bulk_d(i)])
                     return ((uint32_t)fhash(Z.zseed, 0x44454EULL + (uint64_t)pass, (uint64_t)i) & 0xFFFFFF00u) | (uint32_t)i;
                 return 0xFFFFFFFFu;
             });
-            for (int q = 0; q < D && !Z.failed; ++q) Z.dense_cell(M.ord[q]);
+            // the next cell's particle ids in flight while a cell is decided
+            FastZone::Pids next = D > 0 ? Z.load_pids(M.ord[0]) : FastZone::Pids{0, 0, 0, 0};
+            for (int q = 0; q < D && !Z.failed; ++q) {
+                const FastZone::Pids pids = next;
+                if (q + 1 < D) next = Z.load_pids(M.ord[q + 1]);
+                Z.dense_cell(M.ord[q], pids);
+            }
             __syncwarp();
         }
         __syncthreads();
@@ -1724,7 +1773,7 @@ __device__ __forceinline__ void fast_zone_block(int bx, const FastZoneArgs& A, c
         Z.compute_nsm();
         const int L = Z.order_cells([&](int i) -> uint32_t {
             const int cn = Z.cnt(i);
-            if (cn > 0 && (double)cn < Z.low_map(true))
+            if (cn > 0 && cn < A.F.cut[0][1])
                 return ((uint32_t)fhash(Z.zseed, 0x4C4F57ULL, (uint64_t)i) & 0xFFFFFF00u) | (uint32_t)i;
             return 0xFFFFFFFFu;
         });
