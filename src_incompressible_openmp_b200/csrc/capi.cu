@@ -3700,7 +3700,7 @@ int mpcd_learned_grad(const float* features, const float* targets, int64_t rows,
     CUDA_TRY(cudaMemsetAsync(dG, 0, sizeof(float) * kParams, D.stream));
     CUDA_TRY(cudaMemsetAsync(dL, 0, sizeof(float), D.stream));
     CUDA_TRY(cudaMemsetAsync(dS, 0, sizeof(DevStatus), D.stream));
-    k_mlp_grad_tc<<<tg_grid((int)rows, sms), 128, kTgSmem, D.stream>>>(dX, dY, dI, (int)rows, (int)rows,
+    k_mlp_grad_tc<<<tg_grid((int)rows, sms), kTgThreads, kTgSmem, D.stream>>>(dX, dY, dI, (int)rows, (int)rows,
                                                                        1.0f / params[kOffScale], dP, dG, dL, dS);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(grad, dG, sizeof(float) * kParams, cudaMemcpyDeviceToHost, D.stream));
@@ -3752,7 +3752,7 @@ int mpcd_learned_train(const float* features, const float* targets, int64_t rows
             const int64_t r0 = b * batch;
             const int n = (int)std::min<int64_t>(batch, rows - r0);
             ++t;
-            k_mlp_grad_tc<<<tg_grid(n, sms), 128, kTgSmem, D.stream>>>(dX, dY, dI + r0, n, n, yinv, dP, dG, dL + b, dS);
+            k_mlp_grad_tc<<<tg_grid(n, sms), kTgThreads, kTgSmem, D.stream>>>(dX, dY, dI + r0, n, n, yinv, dP, dG, dL + b, dS);
             k_adam<<<(kTrained + 255) / 256, 256, 0, D.stream>>>(dP, dG, dM, dV, kTrained, lr, b1, b2, eps,
                                                                  1.0f - (float)std::pow((double)b1, (double)t),
                                                                  1.0f - (float)std::pow((double)b2, (double)t));

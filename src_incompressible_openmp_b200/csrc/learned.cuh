@@ -568,8 +568,12 @@ __global__ void k_learned_decide(const double* __restrict__ sums, int Nc, double
 }
 
 // ------------------------------------------------------------------ training on the tensor cores
-// Forward and backward of 128-row tiles with tcgen05: one persistent CTA of 128 threads per SM,
-// row t of a tile in thread t (TMEM lane t).
+// Forward and backward of 128-row tiles with tcgen05: one persistent CTA of 512 threads per SM. Row
+// t % 128 of a tile is TMEM lane t % 128 of four threads (one per warpgroup g = t / 128), each of
+// which takes 16 of the 64 hidden units.
+// Bound by the latency of the phases between the MMAs: a training batch of 512 rows is four
+// tiles on four SMs. With one thread per row and all 64 units, uncoalesced weights and rows a
+// batch took 72 us, now 27.
 //   forward:  Z1 = X W1^T (b1 in operand column 75), a1 = bf16(gelu(Z1));
 //             Z2 = A1 W2^T (b2 in operand column 64 of A1), a2 = gelu(Z2); out = W3 a2 + b3 (FP32)
 //   backward: dout = 2 (out - y / scale) / (batch * 2); dW3, db3 in FP32 on the CUDA cores;
@@ -590,10 +594,14 @@ constexpr uint32_t kTgOffD1T = kTgOffD2T + kHid * kTgKR * 2;      // [64][128] b
 constexpr uint32_t kTgOffW1 = kTgOffD1T + kHid * kTgKR * 2;       // [64][80] bf16 (b1 in column 75)
 constexpr uint32_t kTgOffW2 = kTgOffW1 + kHid * kTgK1 * 2;        // [64][80] bf16 (b2 in column 64)
 constexpr uint32_t kTgOffW2T = kTgOffW2 + kHid * kTgK2 * 2;       // [64][64] bf16: W2^T
-constexpr uint32_t kTgOffA2 = kTgOffW2T + kHid * kHid * 2;        // [128][64] f32
-constexpr uint32_t kTgOffDO = kTgOffA2 + 128 * kHid * 4;          // [128][2] f32
+constexpr uint32_t kTgOffA2 = kTgOffW2T + kHid * kHid * 2;        // [128][65] f32
+constexpr int kTgA2 = kHid + 1;                                   // row stride of a2 (bank conflicts)
+constexpr int kTgThreads = 512, kTgGroups = kTgThreads / 128;
+static_assert(kTgGroups * 16 == kHid, "16 hidden units per thread");
+constexpr uint32_t kTgOffDO = kTgOffA2 + 128 * kTgA2 * 4;         // [128][2] f32
 constexpr uint32_t kTgOffW3 = kTgOffDO + 128 * kOut * 4;          // [2][64] f32, b3[2], pad
-constexpr uint32_t kTgOffBar = kTgOffW3 + kOut * kHid * 4 + 16;   // mbarrier
+constexpr uint32_t kTgOffOut = kTgOffW3 + kOut * kHid * 4 + 16;   // [128][2] f32: the output layer
+constexpr uint32_t kTgOffBar = kTgOffOut + 128 * kOut * 4;        // mbarrier
 constexpr uint32_t kTgOffTmem = kTgOffBar + 8;
 constexpr uint32_t kTgSmem = kTgOffTmem + 8;
 constexpr uint32_t kTgTmemCols = 512;
@@ -612,40 +620,46 @@ __device__ __forceinline__ void tg_put(unsigned char* sm, uint32_t off, int r, i
     *reinterpret_cast<__nv_bfloat16*>(sm + off + kmajor_offset(r, k, K)) = __float2bfloat16_rn(v);
 }
 
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(kTgThreads, 1)
     k_mlp_grad_tc(const float* __restrict__ X, const float* __restrict__ Y, const int* __restrict__ idx, int rows,
                   int batch, float yinv, const float* __restrict__ params, float* __restrict__ grad,
                   float* __restrict__ loss, DevStatus* st) {
     extern __shared__ __align__(128) unsigned char sm[];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int row = t & 127, g = t >> 7, h0 = 16 * g;  // this thread's row, warpgroup and first hidden unit
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
     const uint32_t bar = sbase + kTgOffBar;
     float* sA2 = reinterpret_cast<float*>(sm + kTgOffA2);
     float* sDO = reinterpret_cast<float*>(sm + kTgOffDO);
     float* sW3 = reinterpret_cast<float*>(sm + kTgOffW3);
-    // weights (W1 in the point-major operand order of the features), zero padding of the
-    // transposed operands' unused rows
-    for (int i = t; i < kHid * kTgK1; i += 128) {
-        const int n = i / kTgK1, k = i - n * kTgK1;
-        const int pk = (k % 3) * 25 + k / 3;
-        const float w = k < kFeat ? params[kOffW1 + n * kFeat + pk] : (k == kFeat ? params[kOffB1 + n] : 0.0f);
-        tg_put(sm, kTgOffW1, n, k, kTgK1, w);
+    float* sOut = reinterpret_cast<float*>(sm + kTgOffOut);
+    // weights (W1 in the point-major operand order of the features), read in parameter order; the
+    // transposed operands' unused rows stay zero
+#pragma unroll 5
+    for (int i = t; i < kHid * kFeat; i += kTgThreads) {
+        const int n = i / kFeat, pk = i - n * kFeat;
+        tg_put(sm, kTgOffW1, n, 3 * (pk % 25) + pk / 25, kTgK1, params[kOffW1 + i]);
     }
-    for (int i = t; i < kHid * kTgK2; i += 128) {
-        const int n = i / kTgK2, k = i - n * kTgK2;
-        const float w = k < kHid ? params[kOffW2 + n * kHid + k] : (k == kHid ? params[kOffB2 + n] : 0.0f);
+#pragma unroll 4
+    for (int i = t; i < kHid * kHid; i += kTgThreads) {
+        const int n = i / kHid, k = i - n * kHid;
+        const float w = params[kOffW2 + i];
         tg_put(sm, kTgOffW2, n, k, kTgK2, w);
+        tg_put(sm, kTgOffW2T, k, n, kHid, w);  // W2^T[k][n] = W2[n][k]
     }
-    for (int i = t; i < kHid * kHid; i += 128) {
-        const int n = i / kHid, k = i - n * kHid;  // W2^T[n][k] = W2[k][n]
-        tg_put(sm, kTgOffW2T, n, k, kHid, params[kOffW2 + k * kHid + n]);
+    for (int i = t; i < kHid * (kTgK1 - kFeat); i += kTgThreads) {
+        const int n = i / (kTgK1 - kFeat), k = kFeat + i % (kTgK1 - kFeat);
+        tg_put(sm, kTgOffW1, n, k, kTgK1, k == kFeat ? params[kOffB1 + n] : 0.0f);
     }
-    for (int i = t; i < kOut * kHid; i += 128) sW3[i] = bf16r(params[kOffW3 + i]);
+    for (int i = t; i < kHid * (kTgK2 - kHid); i += kTgThreads) {
+        const int n = i / (kTgK2 - kHid), k = kHid + i % (kTgK2 - kHid);
+        tg_put(sm, kTgOffW2, n, k, kTgK2, k == kHid ? params[kOffB2 + n] : 0.0f);
+    }
+    if (t < kOut * kHid) sW3[t] = bf16r(params[kOffW3 + t]);
     if (t < kOut) sW3[kOut * kHid + t] = bf16r(params[kOffB3 + t]);
-    for (int i = t; i < 128 * kTgKR; i += 128) {
-        const int r = i / kTgKR, k = i - r * kTgKR;
-        if (r >= kTgK1 - 4) tg_put(sm, kTgOffXT, r, k, kTgKR, 0.0f);   // operand columns 76..127
-        if (r > kHid) tg_put(sm, kTgOffA1T, r, k, kTgKR, 0.0f);       // columns 65..127
+    for (int i = t; i < 128 * kTgKR / 8; i += kTgThreads) {
+        *reinterpret_cast<uint4*>(sm + kTgOffXT + 16 * i) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(sm + kTgOffA1T + 16 * i) = make_uint4(0u, 0u, 0u, 0u);
     }
     if (t == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
@@ -662,7 +676,7 @@ __global__ void __launch_bounds__(128, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + kTgOffTmem);
-    const uint32_t lb = tmem + ((uint32_t)(warp * 32) << 16);  // this warp's 32 TMEM lanes
+    const uint32_t lb = tmem + ((uint32_t)((warp & 3) * 32) << 16) + h0;  // this warp's lanes, this group's columns
     const float b3a = sW3[kOut * kHid], b3b = sW3[kOut * kHid + 1];
     const float dscale = 2.0f / (float)(batch * kOut);
     const int tiles = (rows + 127) / 128;
@@ -688,74 +702,83 @@ __global__ void __launch_bounds__(128, 1)
         return ok;
     };
     for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const int r = tile * 128 + t;
+        const int r = tile * 128 + row;
         const bool live = r < rows;
         const int src = live ? idx[r] : 0;
-        // 1. the row's operands, row-major and transposed (point-major feature order)
         float y0 = 0.0f, y1 = 0.0f;
         if (live) {
             y0 = Y[(size_t)src * kOut] * yinv;
             y1 = Y[(size_t)src * kOut + 1] * yinv;
         }
-        for (int k = 0; k < kTgK1; ++k) {
-            float v = 0.0f;
-            if (k < kFeat) v = live ? X[(size_t)src * kFeat + (k % 3) * 25 + k / 3] : 0.0f;
-            else if (k == kFeat) v = 1.0f;
-            tg_put(sm, kTgOffX, t, k, kTgK1, v);
-            if (k <= kFeat) tg_put(sm, kTgOffXT, k, t, kTgKR, v);
+        // 1. the rows' operands, row-major and transposed (point-major feature order): a warp reads a
+        // row's 75 features together, 8 rows in turn
+        constexpr int kRowsPerWarp = 128 / (kTgThreads / 32);
+        const int wsrc = __shfl_sync(0xffffffffu, (lane < kRowsPerWarp && tile * 128 + warp * kRowsPerWarp + lane < rows)
+                                                      ? idx[tile * 128 + warp * kRowsPerWarp + lane]
+                                                      : -1, lane);
+#pragma unroll
+        for (int q = 0; q < kRowsPerWarp; ++q) {
+            const int rr = warp * kRowsPerWarp + q;
+            const int sq = __shfl_sync(0xffffffffu, wsrc, q);
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                const int c = lane + 32 * u;  // feature; 75 .. 79: the bias input and padding
+                if (c >= kTgK1) continue;
+                const int k = c < kFeat ? 3 * (c % 25) + c / 25 : c;
+                const float v = c < kFeat ? (sq >= 0 ? X[(size_t)sq * kFeat + c] : 0.0f) : (c == kFeat ? 1.0f : 0.0f);
+                tg_put(sm, kTgOffX, rr, k, kTgK1, v);
+                if (c <= kFeat) tg_put(sm, kTgOffXT, k, rr, kTgKR, v);
+            }
         }
         // 2. Z1 = X W1^T
         if (!sync_mma([&] { tg_mma(tmem, sbase + kTgOffX, sbase + kTgOffW1, kTgK1, false); })) break;
         // 3. a1 = bf16(gelu(Z1)), row-major (column 64: the constant of b2) and transposed
-#pragma unroll
-        for (int h = 0; h < kHid / 16; ++h) {
+        {
             uint32_t z[16];
-            tc_ld16(lb + 16 * h, z);
+            tc_ld16(lb, z);
             tc_ld_wait16(z);
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
                 const float a = gelu(__uint_as_float(z[q]));
-                tg_put(sm, kTgOffA1, t, 16 * h + q, kTgK2, a);
-                tg_put(sm, kTgOffA1T, 16 * h + q, t, kTgKR, a);
+                tg_put(sm, kTgOffA1, row, h0 + q, kTgK2, a);
+                tg_put(sm, kTgOffA1T, h0 + q, row, kTgKR, a);
             }
         }
-        for (int k = kHid; k < kTgK2; ++k) tg_put(sm, kTgOffA1, t, k, kTgK2, k == kHid ? 1.0f : 0.0f);
-        tg_put(sm, kTgOffA1T, kHid, t, kTgKR, 1.0f);
+        if (g == 0) {
+            for (int k = kHid; k < kTgK2; ++k) tg_put(sm, kTgOffA1, row, k, kTgK2, k == kHid ? 1.0f : 0.0f);
+            tg_put(sm, kTgOffA1T, kHid, row, kTgKR, 1.0f);
+        }
         // 4. Z2 = A1 W2^T
         if (!sync_mma([&] { tg_mma(tmem + kHid, sbase + kTgOffA1, sbase + kTgOffW2, kTgK2, false); })) break;
-        // 5. a2, the output layer, dout; dz2 = bf16(dout W3 * gelu'(Z2)), row-major and transposed
-        float o0 = b3a, o1 = b3b;
+        // 5. a2, the output layer (one chain over the hidden units per row and output: group 0 takes
+        // output 0, group 1 output 1), dout; dz2 = bf16(dout W3 * gelu'(Z2)), row-major and transposed
+        uint32_t z2[16];
+        tc_ld16(lb + kHid, z2);
+        tc_ld_wait16(z2);
 #pragma unroll
-        for (int h = 0; h < kHid / 16; ++h) {
-            uint32_t z[16];
-            tc_ld16(lb + kHid + 16 * h, z);
-            tc_ld_wait16(z);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                const int j = 16 * h + q;
-                const float a = gelu(__uint_as_float(z[q]));
-                sA2[t * kHid + j] = a;
-                o0 = fmaf(sW3[j], a, o0);
-                o1 = fmaf(sW3[kHid + j], a, o1);
-            }
+        for (int q = 0; q < 16; ++q) sA2[row * kTgA2 + h0 + q] = gelu(__uint_as_float(z2[q]));
+        __syncthreads();
+        if (g < kOut) {
+            float o = g ? b3b : b3a;
+#pragma unroll 16
+            for (int j = 0; j < kHid; ++j) o = fmaf(sW3[g * kHid + j], sA2[row * kTgA2 + j], o);
+            sOut[kOut * row + g] = o;
         }
+        __syncthreads();
+        const float o0 = sOut[kOut * row], o1 = sOut[kOut * row + 1];
         const float e0 = o0 - y0, e1 = o1 - y1;
         const float d0 = live ? dscale * e0 : 0.0f, d1 = live ? dscale * e1 : 0.0f;
-        if (live) lossAcc += (e0 * e0 + e1 * e1) / (float)(batch * kOut);
-        sDO[2 * t] = d0;
-        sDO[2 * t + 1] = d1;
+        if (g == 0) {
+            if (live) lossAcc += (e0 * e0 + e1 * e1) / (float)(batch * kOut);
+            sDO[2 * row] = d0;
+            sDO[2 * row + 1] = d1;
+        }
 #pragma unroll
-        for (int h = 0; h < kHid / 16; ++h) {
-            uint32_t z[16];
-            tc_ld16(lb + kHid + 16 * h, z);
-            tc_ld_wait16(z);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                const int j = 16 * h + q;
-                const float dz = (d0 * sW3[j] + d1 * sW3[kHid + j]) * gelu_d(__uint_as_float(z[q]));
-                tg_put(sm, kTgOffD2, t, j, kHid, dz);
-                tg_put(sm, kTgOffD2T, j, t, kTgKR, dz);
-            }
+        for (int q = 0; q < 16; ++q) {
+            const int j = h0 + q;
+            const float dz = (d0 * sW3[j] + d1 * sW3[kHid + j]) * gelu_d(__uint_as_float(z2[q]));
+            tg_put(sm, kTgOffD2, row, j, kHid, dz);
+            tg_put(sm, kTgOffD2T, j, row, kTgKR, dz);
         }
         // 6. dA1 = dz2 W2; dW2^T += A1^T dz2
         if (!sync_mma([&] {
@@ -763,56 +786,55 @@ __global__ void __launch_bounds__(128, 1)
                 tg_mma(tmem + 3 * kHid, sbase + kTgOffA1T, sbase + kTgOffD2T, kTgKR, !first);
             }))
             break;
-        // dW3, db3 over the tile's rows (thread i: entry i of W3)
-        {
-            const int o = t / kHid, k = t - o * kHid;
-            float g = 0.0f, gb = 0.0f;
+        // dW3, db3 over the tile's rows (group 0: thread i takes entry i of W3)
+        if (g == 0) {
+            const int o = row / kHid, k = row - o * kHid;
+            float gw = 0.0f, gb = 0.0f;
+#pragma unroll 16
             for (int rr = 0; rr < 128; ++rr) {
                 const float d = sDO[2 * rr + o];
-                g = fmaf(d, sA2[rr * kHid + k], g);
+                gw = fmaf(d, sA2[rr * kTgA2 + k], gw);
                 gb += d;
             }
-            accW3 += g;
+            accW3 += gw;
             if (k == 0) accB3 += gb;
         }
         // 7. dz1 = bf16(dA1 * gelu'(Z1)), transposed
-#pragma unroll
-        for (int h = 0; h < kHid / 16; ++h) {
+        {
             uint32_t z[16], d[16];
-            tc_ld16(lb + 16 * h, z);
-            tc_ld16(lb + 2 * kHid + 16 * h, d);
+            tc_ld16(lb, z);
+            tc_ld16(lb + 2 * kHid, d);
             tc_ld_wait16(z);
             tc_ld_wait16(d);
 #pragma unroll
             for (int q = 0; q < 16; ++q)
-                tg_put(sm, kTgOffD1T, 16 * h + q, t, kTgKR, __uint_as_float(d[q]) * gelu_d(__uint_as_float(z[q])));
+                tg_put(sm, kTgOffD1T, h0 + q, row, kTgKR, __uint_as_float(d[q]) * gelu_d(__uint_as_float(z[q])));
         }
         // 8. dW1^T += X^T dz1 (the wait also frees the operands for the next tile)
         if (!sync_mma([&] { tg_mma(tmem + 4 * kHid, sbase + kTgOffXT, sbase + kTgOffD1T, kTgKR, !first); })) break;
         first = false;
     }
-    // the accumulated gradients: lane t of dW1^T is operand column t (feature, or b1 at 75),
-    // lane t of dW2^T is A1 column t (or b2 at 64)
+    // the accumulated gradients: lane row of dW1^T is an operand column (feature, or b1 at 75), lane
+    // row of dW2^T an A1 column (or b2 at 64)
     if (ok && !first) {
-        const int pk = t < kFeat ? (t % 3) * 25 + t / 3 : -1;
+        const int pk = row < kFeat ? (row % 3) * 25 + row / 3 : -1;
+        uint32_t a[16], b[16];
+        tc_ld16(lb + 4 * kHid, a);
+        tc_ld16(lb + 3 * kHid, b);
+        tc_ld_wait16(a);
+        tc_ld_wait16(b);
 #pragma unroll
-        for (int h = 0; h < kHid / 16; ++h) {
-            uint32_t a[16], b[16];
-            tc_ld16(lb + 4 * kHid + 16 * h, a);
-            tc_ld16(lb + 3 * kHid + 16 * h, b);
-            tc_ld_wait16(a);
-            tc_ld_wait16(b);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                const int j = 16 * h + q;
-                if (t < kFeat) atomicAdd(grad + kOffW1 + j * kFeat + pk, __uint_as_float(a[q]));
-                else if (t == kFeat) atomicAdd(grad + kOffB1 + j, __uint_as_float(a[q]));
-                if (t < kHid) atomicAdd(grad + kOffW2 + j * kHid + t, __uint_as_float(b[q]));
-                else if (t == kHid) atomicAdd(grad + kOffB2 + j, __uint_as_float(b[q]));
-            }
+        for (int q = 0; q < 16; ++q) {
+            const int j = h0 + q;
+            if (row < kFeat) atomicAdd(grad + kOffW1 + j * kFeat + pk, __uint_as_float(a[q]));
+            else if (row == kFeat) atomicAdd(grad + kOffB1 + j, __uint_as_float(a[q]));
+            if (row < kHid) atomicAdd(grad + kOffW2 + j * kHid + row, __uint_as_float(b[q]));
+            else if (row == kHid) atomicAdd(grad + kOffB2 + j, __uint_as_float(b[q]));
         }
-        atomicAdd(grad + kOffW3 + t, accW3);
-        if (t % kHid == 0) atomicAdd(grad + kOffB3 + t / kHid, accB3);
+        if (g == 0) {
+            atomicAdd(grad + kOffW3 + row, accW3);
+            if (row % kHid == 0) atomicAdd(grad + kOffB3 + row / kHid, accB3);
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) lossAcc += __shfl_xor_sync(0xffffffffu, lossAcc, o);
