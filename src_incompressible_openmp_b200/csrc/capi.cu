@@ -115,6 +115,15 @@ struct mpcd_ctx {
     bool srdCellsValid = false;
     CellIndex idxStd, idxSrd;
     bool idxStdValid = false;
+    // The step's shifted pass in place (ZoneArgs::corrSlot): few of its zones change anything, so the
+    // corrected velocities are listed and, in plain steps (shiftPatched), so are the moved particles,
+    // with which the closure reads the pass's input index instead of a new one. Off in a batch that
+    // runs replica by replica.
+    bool shiftInPlace = true;
+    bool shiftPatched = false;
+    int* arrHead = nullptr;      // Nc, -1: list heads of the arrivals (cleared by the closure)
+    uint8_t* depart = nullptr;   // Nc, 0: cells that lost particles (cleared by the closure)
+    int* patchCount = nullptr;   // corrections, movers of the pass (cleared at the start of a step)
     bool idxIota = false;  // the standard index's slots are the identity and not written yet (ensure_std_index)
     uint64_t* blockSums = nullptr;
     uint64_t* blockSumsWalls = nullptr;  // the walls' scan runs beside the index scans
@@ -695,13 +704,15 @@ __device__ __forceinline__ void walls_clear_block(int blk, const BcWork& W, int 
 __global__ void k_walls_clear(BcWork W, int nwords) { walls_clear_block((int)blockIdx.x, W, nwords); }
 
 // The start of a step: block 0 begins it on the device (graph replay) and draws its SRD shift, the
-// others clear the wall bitmaps and counters.
+// others clear the wall bitmaps and counters and the shifted pass's list lengths.
 __global__ void k_step_head(DevParams P, uint64_t seed, const uint64_t* seedDev, long long* stepCounter,
-                            uint64_t* stepSeeds, BcWork W, int nwords) {
-    if (blockIdx.x == 0)
+                            uint64_t* stepSeeds, BcWork W, int nwords, int* patchCount) {
+    if (blockIdx.x == 0) {
         srd_shift_block(P, seed, W.srdShift, seedDev, stepCounter, stepSeeds);
-    else
-        walls_clear_block((int)blockIdx.x - 1, W, nwords);
+        return;
+    }
+    if (blockIdx.x == 1 && threadIdx.x < 2) patchCount[threadIdx.x] = 0;
+    walls_clear_block((int)blockIdx.x - 1, W, nwords);
 }
 
 // the particle state of slots [0, n) from S to T, in one launch
@@ -1067,6 +1078,22 @@ ZoneArgs zone_args(const mpcd_ctx* c, int mode, int xi, int xflip, const uint64_
     return A;
 }
 
+// A with the lists of an in-place pass, in scratch that is free during the shifted pass
+void zone_args_in_place(const mpcd_ctx* c, ZoneArgs& A, bool patched) {
+    A.corrSlot = c->idxSrd.slots;
+    A.corrV = c->vrep;
+    A.corrCount = c->patchCount;
+    if (!patched) return;
+    A.moverSlot = c->idxSrd.pos;
+    A.moverNext = c->idxStd.pos;
+    A.moverCount = c->patchCount + 1;
+    A.arrHead = c->arrHead;
+    A.depart = c->depart;
+}
+RedPatch red_patch(const mpcd_ctx* c, const int* pid) {
+    return RedPatch{c->arrHead, c->depart, c->idxSrd.pos, c->idxStd.pos, c->cidStd, pid};
+}
+
 constexpr int kSms = 148;
 constexpr int kZonesOneWave = 4 * kSms;  // zones that run one per block, all at once
 
@@ -1099,13 +1126,16 @@ int zone_pass_prep(mpcd_ctx* c, int mode, uint64_t seedBase, Prof* pf = nullptr,
     }
     mark(c, pf, 7);
     // velocities out of place (output starts as a copy of the input; zones write what they
-    // change), positions in place (the zone kernel never reads them)
+    // change), positions in place (the zone kernel never reads them); the step's shifted pass keeps
+    // the velocities in place too and lists its changes
+    const bool inPlace = inStep && shiftedPass && c->shiftInPlace;
     const int xi = c->xv, xo = c->xv ^ 1;
-    if (c->n > 0) {
+    if (c->n > 0 && !inPlace) {
         WITH_VIEWS(xi, xo, k_copy_vel<<<blocks_for(c->n), kThreads, 0, c->stream>>>(S, T, c->n));
         ++c->launches;
     }
     ZoneArgs A = zone_args(c, mode, xi, c->xflip, seeds);
+    if (inPlace) zone_args_in_place(c, A, c->shiftPatched);
     // heaviest zones first (by estimated dense-phase work) in the base pass; the shifted pass
     // runs after the base pass has evened the counts, its zones cost about the same, and the
     // two ordering kernels would cost more than the tail they save
@@ -1167,11 +1197,15 @@ OverflowJob overflow_job(const mpcd_ctx* c, bool metrics) {
     return overflow_job(c, c->zA, metrics ? c->passOut + (c->zMode == MPCD_LAYOUT_SHIFTED ? 4 : 0) : nullptr);
 }
 
-// host-side state after a pass: velocities in the other buffer, positions in place
+// host-side state after a pass: velocities in the other buffer (unless in place), positions in place
 void zone_pass_flip(mpcd_ctx* c) {
-    c->xv ^= 1;
-    c->xflip ^= 1;
-    c->idxStdValid = false;  // cid was updated for moved particles; positions changed
+    if (!c->zA.corrSlot) {
+        c->xv ^= 1;
+        c->xflip ^= 1;
+    }
+    // cid was updated for moved particles; positions changed. A patched pass leaves its input's index
+    // to the closure.
+    c->idxStdValid = c->zA.moverSlot != nullptr;
     c->srdCellsValid = false;
 }
 
@@ -1182,6 +1216,11 @@ int zone_pass_finish(mpcd_ctx* c, Prof* pf = nullptr, bool metrics = true) {
     else
         k_zone_overflow<false><<<c->ovBlocks, 32, 0, c->stream>>>(J.A, J.gmem, J.perBlock, J.blocksDone, J.metricsOut);
     ++c->launches;
+    if (c->zA.corrSlot) {
+        WITH_VIEW(c->xv, k_apply_corr<<<std::min(blocks_for(c->n), 2 * kSms), kThreads, 0, c->stream>>>(
+                             S, c->zA.corrSlot, c->zA.corrV, c->zA.corrCount));
+        ++c->launches;
+    }
     CUDA_TRY(cudaGetLastError());
     mark(c, pf, 8);
     zone_pass_flip(c);
@@ -1302,11 +1341,13 @@ int run_closure(mpcd_ctx* c, bool permute, bool wantRep, bool wantStats, Prof* p
     if (learned || c->sampling) {  // the stencil features read the red fields
         rf.feat = c->redFeat;
     }
+    const bool patched = permute && c->shiftPatched;  // the shifted pass's input index, with its patches
     // the step's fast path; learned steps always take it (their closure has no diagnostics)
     const bool flat = permute && (learned || (!wantRep && !wantStats));
     WITH_VIEW(c->xv, k_closure_cells<<<blocks_for(c->Nc), kThreads, 0, c->stream>>>(
                          c->P, c->idxStd.start, c->idxStd.slots, S, c->refPx, c->refPy, c->refUx, c->refUy, rf, c->duRX,
-                         c->duRY, c->cols, flat ? c->cellOf : nullptr));
+                         c->duRY, c->cols, flat ? c->cellOf : nullptr,
+                         patched ? red_patch(c, c->pidb[c->pp]) : RedPatch{}));
     ++c->launches;
     rc = reduce_cols(c, c->cols, c->Nc, 2, 0u, c->red);
     if (rc) return rc;
@@ -1352,6 +1393,7 @@ int run_closure(mpcd_ctx* c, bool permute, bool wantRep, bool wantStats, Prof* p
         c->pp ^= 1;
         c->slotsSorted = true;
         c->idxIota = true;
+        if (patched) c->idxStdValid = false;  // the few moved particles lie in their old cells' runs
         mark(c, pf, 10);
         // the standard index stays valid (same cells, identity slots); per-slot cell ids and
         // SRD cells refer to the old layout
@@ -1396,7 +1438,7 @@ int mpcd_ctx_destroy(mpcd_ctx* c) {
                     c->idxSrd.count, c->idxSrd.start, c->idxSrd.pos, c->idxSrd.slots,
                     c->blockSums, c->blockSumsWalls, c->W.bitsX, c->W.bitsY, c->W.wordCount, c->W.wordPrefix, c->W.events,
                     c->W.nEvents, c->W.normals, c->W.contrib, c->W.blockPartial, c->W.ints, c->W.srdShift,
-                    c->wallOut, c->signs, c->seeds, c->seedsShifted, c->zoneMoved, c->zoneCorr, c->overflow, c->nOverflow, c->ovDone,
+                    c->wallOut, c->signs, c->seeds, c->seedsShifted, c->arrHead, c->depart, c->patchCount, c->zoneMoved, c->zoneCorr, c->overflow, c->nOverflow, c->ovDone,
                     c->zoneCost, c->zoneHist, c->zoneOrder, c->dStep, c->stepSeeds,
                     c->slotsLive, c->liveCnt, c->liveStart, c->liveTop, c->duScratch, c->zkRect, c->zkDiag, c->zkOut,
                     c->lparams, c->lmode, c->lcount, c->lsums, c->duLX, c->duLY, c->duLSum, c->redFeat,
@@ -1568,6 +1610,12 @@ int mpcd_ctx_create_form(const mpcd_params_c* params, int device, int32_t form, 
                 return fail(set_err(MPCD_ERR_CUDA, "seed events"));
         }
     }
+    ALLOC(c->arrHead, (size_t)Nc);
+    ALLOC(c->depart, (size_t)Nc);
+    ALLOC(c->patchCount, 2);
+    if (cudaMemset(c->arrHead, 0xFF, sizeof(int) * (size_t)Nc) != cudaSuccess ||
+        cudaMemset(c->depart, 0, (size_t)Nc) != cudaSuccess || cudaMemset(c->patchCount, 0, 2 * sizeof(int)) != cudaSuccess)
+        return fail(set_err(MPCD_ERR_CUDA, "shifted-pass patches"));
     ALLOC(c->zoneMoved, (size_t)maxZones);
     ALLOC(c->zoneCorr, (size_t)maxZones);
     ALLOC(c->overflow, (size_t)maxZones);
@@ -2328,7 +2376,7 @@ static int step_head(mpcd_ctx* c, int64_t step, bool metrics, Prof* pf) {
     mark(c, pf, -1);
     k_step_head<<<1 + blocks_for(c->nwords), kThreads, 0, c->stream>>>(
         c->P, 130363ULL + 10007ULL * s, c->graphMode ? c->stepSeeds : nullptr, c->graphMode ? c->dStep : nullptr,
-        c->stepSeeds, c->W, c->nwords);
+        c->stepSeeds, c->W, c->nwords, c->patchCount);
     ++c->launches;
     CUDA_TRY(cudaGetLastError());
     if (c->seedsEarly) {
@@ -2434,11 +2482,15 @@ static int step_tail(mpcd_ctx* c, bool metrics, Prof* pf) {
 }
 
 static int step_once(mpcd_ctx* c, int64_t step, bool metrics, Prof* pf = nullptr) {
+    // Metrics rows and the learned closure read the red state's index; the mean-flow removal adds up
+    // the velocities in slot order, which a patched step leaves slightly out of cell order.
+    c->shiftPatched = c->shiftInPlace && !metrics && !c->learnedOn && !c->sampling && !c->P.keepMeanFlow;
     int rc = step_head(c, step, metrics, pf);
     if (!rc) rc = zone_pass_kernel(c);
     if (!rc) rc = step_mid(c, step, metrics, pf);
     if (!rc) rc = zone_pass_kernel(c);
     if (!rc) rc = step_tail(c, metrics, pf);
+    c->shiftPatched = false;
     return rc;
 }
 
@@ -3030,7 +3082,7 @@ static int batch_status(mpcd_batch* b) {
 // replica's zone_pass_prep has filled its zA
 static int batch_zone_kernel(mpcd_batch* b, int pass) {
     const int n = (int)b->members.size();
-    const int slot = (b->members[0]->xv & 1) * 2 + pass;
+    const int slot = ((b->members[0]->xv & 1) * 2 + (b->members[0]->xflip & 1)) * 2 + pass;
     ZoneArgs* h = b->hArgs + (size_t)slot * n;
     int* ho = b->hOffs + (size_t)slot * (n + 1);
     ho[0] = 0;
@@ -3092,7 +3144,7 @@ static int batch_index(mpcd_batch* b) {
 // the batched zone kernel), then each replica's host-side flip; staged like the zone arguments
 static int batch_zone_finish(mpcd_batch* b, int pass) {
     const int n = (int)b->members.size();
-    const int slot = (b->members[0]->xv & 1) * 2 + pass;
+    const int slot = ((b->members[0]->xv & 1) * 2 + (b->members[0]->xflip & 1)) * 2 + pass;
     OverflowJob* h = b->hOv + (size_t)slot * n;
     for (int r = 0; r < n; ++r) h[r] = overflow_job(b->members[r], false);
     OverflowJob* d = b->dOv + (size_t)slot * n;
@@ -3110,6 +3162,16 @@ static int batch_zone_finish(mpcd_batch* b, int pass) {
 // is small enough for the one-block scan and all share a particle-id buffer parity, the
 // standard-grid index builds that follow each pass.
 static int batch_step_body(mpcd_batch* b, int64_t step) {
+    // out-of-place passes: their arguments are staged per buffer orientation
+    struct OutOfPlace {
+        mpcd_batch* b;
+        explicit OutOfPlace(mpcd_batch* q) : b(q) {
+            for (mpcd_ctx* c : b->members) c->shiftInPlace = false;
+        }
+        ~OutOfPlace() {
+            for (mpcd_ctx* c : b->members) c->shiftInPlace = true;
+        }
+    } guard(b);
     bool idx = b->indexBatched;
     for (mpcd_ctx* c : b->members) idx = idx && c->pp == b->members[0]->pp;
     int rc = batch_each(b, [&](mpcd_ctx* c) { return step_head(c, step, false, nullptr); });
@@ -3265,9 +3327,9 @@ int mpcd_batch_create(const mpcd_params_c* params, int count, int device, mpcd_b
         return set_err(MPCD_ERR_CUDA, "batch stream");
     }
     {
-        // staging of the batched zone kernels (4 slots: buffer parity x pass), the shared
+        // staging of the batched zone kernels (8 slots: velocity and position buffer x pass), the shared
         // memory of the largest working set plus the arguments, the step counters
-        const size_t nslots = 4;
+        const size_t nslots = 8;
         std::vector<long long*> steps((size_t)count);
         for (int r = 0; r < count; ++r) {
             b->zSmem = std::max(b->zSmem, b->members[r]->zSmem + (size_t)kZoneArgsSmem);

@@ -85,6 +85,16 @@ struct RedFields {
     double *Px, *Py, *Ux, *Uy;
     float4* feat;  // (N/gamma - 1, Ux, Uy, N) as FP32: the learned closure's stencil input
 };
+// The red state of a step whose shifted pass ran in place: `start` and `slots` are still the pass's
+// input index, and the few particles that changed cells are listed per new cell, with a flag per old
+// cell (ZoneArgs::arrHead ...). arrHead nullptr: the index is the red state's own. The lists and flags
+// are cleared as they are read. (An index rebuilt for at most a few moves per zone took 1.24 ms at
+// 84 M particles, the copy of the velocities for an out-of-place pass 0.40 ms.)
+struct RedPatch {
+    int* arrHead;
+    uint8_t* depart;
+    const int *moverSlot, *moverNext, *cid, *pid;
+};
 template <class V>
 __device__ __forceinline__ void closure_cells_block(int blk, const DevParams& P, const uint64_t* __restrict__ start,
                                                     const int* __restrict__ slots, const V& S,
@@ -92,17 +102,55 @@ __device__ __forceinline__ void closure_cells_block(int blk, const DevParams& P,
                                                     const double* __restrict__ refUx, const double* __restrict__ refUy,
                                                     const RedFields& red, double* __restrict__ duRX,
                                                     double* __restrict__ duRY, double* __restrict__ cols,
-                                                    int* __restrict__ cellOf) {
+                                                    int* __restrict__ cellOf, const RedPatch& patch) {
     const int c = blk * blockDim.x + threadIdx.x;
     if (c >= P.Nc) return;
     const int a = (int)(uint32_t)start[c], b = (int)(uint32_t)start[c + 1];
-    const int m = b - a;
+    int m = b - a;
     double px = 0.0, py = 0.0;
-    for (int j = a; j < b; ++j) {
-        const double2 w = S.vel(slots[j]);
-        px = __dadd_rn(px, w.x);
-        py = __dadd_rn(py, w.y);
-        if (cellOf) cellOf[j] = c;
+    const int head = patch.arrHead ? patch.arrHead[c] : -1;
+    if (head < 0 && !(patch.arrHead && patch.depart[c])) {
+        for (int j = a; j < b; ++j) {
+            const double2 w = S.vel(slots[j]);
+            px = __dadd_rn(px, w.x);
+            py = __dadd_rn(py, w.y);
+            if (cellOf) cellOf[j] = c;
+        }
+    } else {
+        // the members that stayed (ascending particle id) merged with the arrivals
+        patch.arrHead[c] = -1;
+        patch.depart[c] = 0;
+        m = 0;
+        int last = -1;  // id of the last arrival added
+        auto add = [&](int s) {
+            const double2 w = S.vel(s);
+            px = __dadd_rn(px, w.x);
+            py = __dadd_rn(py, w.y);
+            ++m;
+        };
+        auto arrivals_below = [&](int limit) {
+            for (;;) {
+                int best = limit, at = -1;
+                for (int k = head; k >= 0; k = patch.moverNext[k]) {
+                    const int s = patch.moverSlot[k], q = patch.pid[s];
+                    if (q > last && q < best) {
+                        best = q;
+                        at = s;
+                    }
+                }
+                if (at < 0) return;
+                add(at);
+                last = best;
+            }
+        };
+        for (int j = a; j < b; ++j) {
+            const int s = slots[j], now = patch.cid[s];
+            if (cellOf) cellOf[j] = now;
+            if (now != c) continue;
+            arrivals_below(patch.pid[s]);
+            add(s);
+        }
+        arrivals_below(0x7fffffff);
     }
     double ux = 0.0, uy = 0.0;
     if (m > 0) {
@@ -128,8 +176,22 @@ __global__ void k_closure_cells(DevParams P, const uint64_t* __restrict__ start,
                                 const double* __restrict__ refPx,
                                 const double* __restrict__ refPy, const double* __restrict__ refUx,
                                 const double* __restrict__ refUy, RedFields red, double* __restrict__ duRX,
-                                double* __restrict__ duRY, double* __restrict__ cols, int* __restrict__ cellOf) {
-    closure_cells_block((int)blockIdx.x, P, start, slots, S, refPx, refPy, refUx, refUy, red, duRX, duRY, cols, cellOf);
+                                double* __restrict__ duRY, double* __restrict__ cols, int* __restrict__ cellOf,
+                                RedPatch patch) {
+    closure_cells_block((int)blockIdx.x, P, start, slots, S, refPx, refPy, refUx, refUy, red, duRX, duRY, cols, cellOf,
+                        patch);
+}
+
+// the corrected velocities of an in-place zone pass into the state
+template <class V>
+__device__ __forceinline__ void apply_corr_block(int blk, int nblk, const V& S, const int* __restrict__ slot,
+                                                 const double2* __restrict__ v, const int* __restrict__ count) {
+    const int n = *count;
+    for (int i = blk * (int)blockDim.x + (int)threadIdx.x; i < n; i += nblk * (int)blockDim.x) S.set_vel(slot[i], v[i]);
+}
+template <class V>
+__global__ void k_apply_corr(V S, const int* __restrict__ slot, const double2* __restrict__ v, const int* __restrict__ count) {
+    apply_corr_block((int)blockIdx.x, (int)gridDim.x, S, slot, v, count);
 }
 
 // ---------------------------------------------------------------- fixed-order reductions

@@ -19,8 +19,12 @@ namespace mpcd_dev {
 struct F64Job {
     DevParams P;
     View64 S;          // the state at the step's start (velocities of the base pass's input)
-    View64 M;          // after the base pass (the same positions)
+    View64 M;          // after the base pass (the same positions); the shifted pass runs on it in place
     View64 T;          // the step's result
+    RedPatch patch;    // the shifted pass's moves
+    int* patchCount;
+    const int* corrSlot;
+    const double2* corrV;
     const int* pid;
     int* pidOut;
     int* cidStd;
@@ -45,7 +49,7 @@ struct F64Job {
 constexpr int kF64CollideShape = 0;     // 32 cells by 128 threads (the tuner's usual choice)
 constexpr int kF64CollideCells = kCollideShape[kF64CollideShape].cells;
 constexpr int kF64CollideThreads = kCollideShape[kF64CollideShape].threads;
-constexpr int kF64WallBlocks = 8;       // blocks per replica of the thermal-wall kernel
+constexpr int kF64WallBlocks = 8;       // blocks per replica of the thermal-wall and correction kernels
 
 #define MPCD_F64_JOB(J, blk)                                            \
     __shared__ __align__(16) char sj[fb_bytes<F64Job>()];               \
@@ -71,6 +75,7 @@ __global__ void __launch_bounds__(256) k_f64_head(F64Jobs jobs, F64Offs offs, in
     }
     if (i < 4) J.W.ints[i] = 0;
     if (i == 0) *J.W.nEvents = 0;
+    if (i < 2) J.patchCount[i] = 0;
 }
 
 // zone generators of the base, then the shifted pass
@@ -147,15 +152,17 @@ __global__ void __launch_bounds__(256) k_f64_eos(F64Jobs jobs, F64Offs offs, int
     eos_block(blk, J.P, J.pdrive, J.eosX, J.eosY);
 }
 
-// the pass's output velocities start as a copy of its input: base S -> M, shifted M -> S
-__global__ void __launch_bounds__(256) k_f64_copy_vel(F64Jobs jobs, F64Offs offs, int n, int shifted) {
+// the base pass's output velocities start as a copy of its input
+__global__ void __launch_bounds__(256) k_f64_copy_vel(F64Jobs jobs, F64Offs offs, int n) {
     MPCD_F64_JOB(J, blk);
     const int i = blk * (int)blockDim.x + (int)threadIdx.x;
-    if (i >= J.n) return;
-    if (shifted)
-        J.S.v[i] = J.M.v[i];
-    else
-        J.M.v[i] = J.S.v[i];
+    if (i < J.n) J.M.v[i] = J.S.v[i];
+}
+// the shifted pass's corrected velocities
+__global__ void __launch_bounds__(256) k_f64_apply_corr(F64Jobs jobs) {
+    __shared__ __align__(16) char sj[fb_bytes<F64Job>()];
+    const F64Job& J = fb_stage(jobs, (int)blockIdx.x / kF64WallBlocks, sj);
+    apply_corr_block((int)blockIdx.x % kF64WallBlocks, kF64WallBlocks, J.M, J.corrSlot, J.corrV, J.patchCount);
 }
 
 __global__ void __launch_bounds__(256) k_f64_zone_cost(F64Jobs jobs, F64Offs offs, int n) {
@@ -170,8 +177,8 @@ __global__ void __launch_bounds__(1024) k_f64_zone_order(F64Jobs jobs) {
 
 __global__ void __launch_bounds__(256) k_f64_closure(F64Jobs jobs, F64Offs offs, int n) {
     MPCD_F64_JOB(J, blk);
-    closure_cells_block(blk, J.P, J.startStd, J.slotsStd, J.S, J.ref.Px, J.ref.Py, J.ref.Ux, J.ref.Uy, RedFields{}, J.duRX,
-                        J.duRY, J.cols, J.cellOf);
+    closure_cells_block(blk, J.P, J.startStd, J.slotsStd, J.M, J.ref.Px, J.ref.Py, J.ref.Ux, J.ref.Uy, RedFields{}, J.duRX,
+                        J.duRY, J.cols, J.cellOf, J.patch);
 }
 __global__ void __launch_bounds__(kRedThreads) k_f64_reduce_partial(F64Jobs jobs, F64Offs offs, int n) {
     __shared__ double sh[2][kRedThreads];
@@ -186,7 +193,7 @@ __global__ void __launch_bounds__(kRedThreads) k_f64_reduce_final(F64Jobs jobs) 
 }
 __global__ void __launch_bounds__(256) k_f64_kick(F64Jobs jobs, F64Offs offs, int n) {
     MPCD_F64_JOB(J, blk);
-    kick_flat_block(blk, J.P, J.n, J.cellOf, J.slotsStd, J.red, J.duRX, J.duRY, J.eosX, J.eosY, J.S, J.pid, J.T, J.pidOut,
+    kick_flat_block(blk, J.P, J.n, J.cellOf, J.slotsStd, J.red, J.duRX, J.duRY, J.eosX, J.eosY, J.M, J.pid, J.T, J.pidOut,
                     nullptr, nullptr, nullptr, nullptr);
 }
 

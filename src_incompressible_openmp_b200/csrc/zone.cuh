@@ -82,6 +82,17 @@ struct ZoneArgs {
     // vin, xout, vout are unused
     int f32;
     View32 in32, out32;
+    // in-place pass (the step's shifted pass; corrSlot nullptr otherwise): corrected velocities go to
+    // a list (slot, velocity), written to the input's velocities after the pass (k_apply_corr); at
+    // most one entry per particle, since a particle has one owner zone and one final cell
+    int* corrSlot;
+    double2* corrV;
+    int* corrCount;
+    // the particles that changed cells in it (moverSlot nullptr: not wanted), as a list per new cell
+    // (arrHead, moverNext; -1 ends it) and a flag per old cell: the closure then reads the index of
+    // the pass's input with these patches
+    int *moverSlot, *moverNext, *moverCount, *arrHead;
+    uint8_t* depart;
 };
 
 // pass input / output velocities of slot s (kF32: the FP32 views, instantiated separately)

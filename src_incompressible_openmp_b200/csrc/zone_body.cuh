@@ -1341,6 +1341,22 @@ __device__ __forceinline__ bool zone_finish(ZoneState<I, kF32>& S, const ZoneArg
                 }
             }
         };
+        if (!kSerial && mat && A.moverSlot) {
+            // the particles of this list that changed cells (a list left implicit has none)
+#pragma unroll 1
+            for (int j = 0; j < n; ++j) {
+                const uint32_t e = M.arena[at + j];
+                const int lc = (int)(e >> kEntryShift);
+                if (!(M.cflags[lc] & kCOwned)) continue;
+                const int sl = A.slots[M.gstart[lc] + (int)(e & ((1u << kEntryShift) - 1))];
+                const int from = S.gy_of(lc) + p.Ny * S.gx_of(lc), to = A.cid[sl];
+                if (to == from) continue;
+                const int m = atomicAdd(A.moverCount, 1);
+                A.moverSlot[m] = sl;
+                A.moverNext[m] = atomicExch(A.arrHead + to, m);
+                A.depart[from] = 1;
+            }
+        }
         double bx = 0.0, by = 0.0, axs = 0.0, ays = 0.0;
         sum((int)M.cnt0[l], [&](int j) { return A.slots[g0 + j]; }, bx, by);
         sum(n, [&](int j) {
@@ -1370,6 +1386,24 @@ __device__ __forceinline__ bool zone_finish(ZoneState<I, kF32>& S, const ZoneArg
         if (kSerial) {
             // in place: every cell's sums must read the velocities of the zone's start
             if (doCorr) A.duScratch[l] = make_double2(ux, uy);
+        } else if (doCorr && A.corrSlot) {  // in place: listed (few cells: one entry at a time)
+            if (mat || (f & kCOwned)) {
+                int k = n;
+                if (mat) {
+                    k = 0;
+#pragma unroll 1
+                    for (int j = 0; j < n; ++j) k += !(M.arena[at + j] >> 31);
+                }
+                int d = k > 0 ? atomicAdd(A.corrCount, k) : 0;
+#pragma unroll 1
+                for (int j = 0; j < n; ++j) {
+                    const int sl = mat ? (int)M.arena[at + j] : A.slots[at + j];
+                    if (sl < 0) continue;
+                    const double2 w = zone_vin<kF32>(A, sl);
+                    A.corrSlot[d] = sl;
+                    A.corrV[d++] = make_double2(__dadd_rn(w.x, ux), __dadd_rn(w.y, uy));
+                }
+            }
         } else if (doCorr && (mat || (f & kCOwned))) {
             for (int j0 = 0; j0 < n; j0 += 8) {
                 int sl[8];
