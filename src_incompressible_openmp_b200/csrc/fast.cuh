@@ -2089,19 +2089,27 @@ __device__ __forceinline__ double2 fast_position(const DevParams& P, int ix, int
     return make_double2(((double)ix + (double)o.x) * P.dx, ((double)iy + (double)o.y) * P.dy);
 }
 
-// the bins into FP64 positions and velocities in particle-id order (each nullable)
-__global__ void k_fast_store(DevParams P, FastParams F, FastBins b, double2* __restrict__ x, double2* __restrict__ v) {
+// a stored velocity with its cell's pending closure kick
+__device__ __forceinline__ float2 fast_kicked(float2 w, int2 k) {
+    return make_float2(fv_of(fq_of(w.x) + k.x), fv_of(fq_of(w.y) + k.y));
+}
+
+// the bins into FP64 positions and velocities in particle-id order (each nullable), the pending kick
+// (nullable) added on the way
+__global__ void k_fast_store(DevParams P, FastParams F, FastBins b, const int2* __restrict__ kick, double2* __restrict__ x,
+                             double2* __restrict__ v) {
     const int c = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (c >= P.Nc) return;
     const int n = min(b.cnt[c], F.K);
     const int ix = c / P.Ny, iy = c - ix * P.Ny;
+    const int2 kq = kick ? kick[c] : make_int2(0, 0);
     for (int j = lane; j < n; j += 32) {
         const size_t s = (size_t)c * F.K + j;
         const int p = b.pid[s];
         if (p < 0 || p >= P.n) continue;
         const float2 o = b.off[s];
-        const float2 w = b.vel[s];
+        const float2 w = fast_kicked(b.vel[s], kq);
         if (x) x[p] = fast_position(P, ix, iy, o);
         if (v) v[p] = make_double2((double)w.x, (double)w.y);
     }

@@ -98,9 +98,9 @@ __global__ void __launch_bounds__(256) k_fb_begin(const FastBeginJob* __restrict
     if (c < J.Nc) J.cntOut[c] = 0;
 }
 
-// before the first step of a call: the pending kicks into the bins (pending), the kick arrays to
-// zero, the step counters to step0. A warp takes the cells of its 32 threads one after another.
-// (A flush, a copy, a fill and a synchronisation per member took 15 ms at 256 replicas.)
+// before the first step of a call: the step counters to step0 and, where no kick is pending, the kick
+// arrays to zero (every batched stream applies them). (A flush, a copy, a fill and a synchronisation
+// per member took 15 ms at 256 replicas.)
 __global__ void __launch_bounds__(256) k_fb_enter(const FastStreamJob* __restrict__ jobs, const int* __restrict__ offs, int n,
                                                   long long step0, int pending) {
     __shared__ __align__(16) char sj[fb_bytes<FastStreamJob>()];
@@ -109,24 +109,8 @@ __global__ void __launch_bounds__(256) k_fb_enter(const FastStreamJob* __restric
     const FastStreamJob& J = fb_stage(jobs, r, sj);
     const int blk = (int)blockIdx.x - offs[r];
     if (blk == 0 && threadIdx.x == 0) J.S->step = step0;
-    const int c = blk * (int)blockDim.x + (int)threadIdx.x, lane = threadIdx.x & 31;
-    int2 kq = make_int2(0, 0);
-    int cnt = 0;
-    if (c < J.P.Nc) {
-        kq = J.kick[c];
-        J.kick[c] = make_int2(0, 0);
-        if (kq.x != 0 || kq.y != 0) cnt = min(J.in.cnt[c], J.F.K);
-    }
-    if (!pending) return;
-    for (int k = 0; k < 32; ++k) {
-        const int m = __shfl_sync(0xffffffffu, cnt, k);
-        const int kx = __shfl_sync(0xffffffffu, kq.x, k), ky = __shfl_sync(0xffffffffu, kq.y, k);
-        const size_t base = (size_t)(c - lane + k) * J.F.K;
-        for (int j = lane; j < m; j += 32) {
-            const float2 v = J.in.vel[base + j];
-            J.in.vel[base + j] = make_float2(fv_of(fq_of(v.x) + kx), fv_of(fq_of(v.y) + ky));
-        }
-    }
+    const int c = blk * (int)blockDim.x + (int)threadIdx.x;
+    if (!pending && c < J.P.Nc) J.kick[c] = make_int2(0, 0);
 }
 
 __global__ void __launch_bounds__(256, 4) k_fb_stream(const FastStreamJob* __restrict__ jobs, const int* __restrict__ offs,

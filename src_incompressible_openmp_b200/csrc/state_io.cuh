@@ -97,8 +97,10 @@ __global__ void __launch_bounds__(kPartThreads) k_part_slots(const double2* __re
     });
 }
 
-// The fast form's bins into the buckets: a block takes cellsPer (at most kPartThreads) cells.
-__global__ void __launch_bounds__(kPartThreads) k_part_bins(DevParams P, FastParams F, FastBins b, int cellsPer, int shift,
+// The fast form's bins into the buckets: a block takes cellsPer (at most kPartThreads) cells; the
+// pending kick (nullable) is added on the way.
+__global__ void __launch_bounds__(kPartThreads) k_part_bins(DevParams P, FastParams F, FastBins b,
+                                                            const int2* __restrict__ kick, int cellsPer, int shift,
                                                             PartBuf B) {
     __shared__ int start[kPartThreads + 1];
     __shared__ uint64_t scan[32];
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(kPartThreads) k_part_bins(DevParams P, FastPar
             const size_t s = (size_t)c * F.K + (f - start[g]);
             p = b.pid[s];
             X = fast_position(P, ix, iy, b.off[s]);
-            const float2 w = b.vel[s];
+            const float2 w = fast_kicked(b.vel[s], kick ? kick[c] : make_int2(0, 0));
             V = make_double2((double)w.x, (double)w.y);
         });
 }
