@@ -110,7 +110,6 @@ struct mpcd_ctx {
     uint64_t* sortKeysSide = nullptr;  // n
     cudaEvent_t stdIdxDone = nullptr;
     bool stdIdxPending = false;
-    int rankCells = 1;             // cells per block of k_cell_rank
     bool cidStdValid = false;
     bool srdCellsValid = false;
     CellIndex idxStd, idxSrd;
@@ -679,7 +678,7 @@ int build_index(mpcd_ctx* c, const int* cid, CellIndex& I, Prof* pf = nullptr, i
     if (c->n > 0) {
         k_scatter_keys<<<blocks_for(c->n, kThreads * kIndexItems), kThreads, 0, s>>>(
             cid, I.pos, c->pidb[c->pp], c->n, I.start, keys); ++c->launches;
-        k_cell_rank<<<blocks_for(c->Nc, c->rankCells), kRankThreads, 0, s>>>(I.start, c->Nc, c->rankCells, keys,
+        k_cell_rank<<<blocks_for(c->Nc, kRankCells), kRankThreads, 0, s>>>(I.start, c->Nc, keys,
                                                                             I.slots); ++c->launches;
     }
     CUDA_TRY(cudaGetLastError());
@@ -1535,7 +1534,6 @@ int mpcd_ctx_create_form(const mpcd_params_c* params, int device, int32_t form, 
     ALLOC(c->cidSrd, (size_t)n);
     ALLOC(c->sortKeys, (size_t)n);
     ALLOC(c->sortKeysSide, (size_t)n);
-    c->rankCells = rank_cells_per_block(n, Nc);
     for (CellIndex* I : {&c->idxStd, &c->idxSrd}) {
         ALLOC(I->count, (size_t)Nc);
         if (cudaMemset(I->count, 0, sizeof(int) * (size_t)std::max(Nc, 1)) != cudaSuccess)
@@ -3369,7 +3367,7 @@ int mpcd_batch_create(const mpcd_params_c* params, int count, int device, mpcd_b
         for (mpcd_ctx* c : b->members) {
             b->indexBatched = b->indexBatched && c->Nc <= kSmallScan;
             oh.push_back(oh.back() + (c->n > 0 ? blocks_for(c->n, kThreads * kIndexItems) : 0));
-            orank.push_back(orank.back() + blocks_for(c->Nc, c->rankCells));
+            orank.push_back(orank.back() + blocks_for(c->Nc, kRankCells));
         }
         b->histBlocks = oh.back();
         b->rankBlocks = orank.back();
@@ -3382,7 +3380,7 @@ int mpcd_batch_create(const mpcd_params_c* params, int count, int device, mpcd_b
             for (mpcd_ctx* c : b->members) {
                 CellIndex& I = c->idxStd;
                 jobs.push_back(IndexJob{c->cidStd, I.count, I.pos, I.start, I.slots, c->pidb[q], c->sortKeys, c->n,
-                                        c->Nc, c->rankCells});
+                                        c->Nc});
             }
             ok = cudaMalloc((void**)&b->dJobs[q], sizeof(IndexJob) * jobs.size()) == cudaSuccess &&
                  cudaMemcpy(b->dJobs[q], jobs.data(), sizeof(IndexJob) * jobs.size(), cudaMemcpyHostToDevice) ==

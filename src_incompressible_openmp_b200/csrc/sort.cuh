@@ -7,8 +7,8 @@
 //
 // Build: warp-aggregated histogram with atomics (one atomic per run of equal cell ids in a
 // warp), exclusive scan of the counts, scatter of (particle id, slot) keys into the cells'
-// segments, then a rank sort of each tile of cells in shared memory: an entry's place in its
-// cell is the number of the cell's keys below its own.
+// segments, then a rank sort of each cell's keys: an entry's place in its cell is the number of the
+// cell's keys below its own.
 #pragma once
 
 #include "common.cuh"
@@ -259,90 +259,128 @@ __global__ void k_scatter_keys(const int* __restrict__ cid, const int* __restric
     scatter_keys_block((int)blockIdx.x, cid, pos, pid, n, start, keys);
 }
 
+// Rank sort of the cells' keys. Eight lanes take a cell of up to 32 entries: their keys stay in
+// registers, the cell's ids go through shared memory and are read four at a time, and no block barrier
+// is needed; K registers per lane by the fullest such cell of the warp. Larger cells take the whole
+// warp. Bound by the latency of start, then keys, and by the m^2 comparisons of a cell (about 400 at 20
+// entries). At 84 M particles, 20 per cell, a whole index build took 1.24 ms with a block's ~1,280 keys
+// and their segment bounds in shared memory, a thread per key and two barriers, and 1.07-1.11 ms so
+// (0.17 -> 0.16 ms at 10.5 M, 10 per cell; 0.024 -> 0.019 ms at 2,500 cells). Sixteen cells per warp:
+// 1.13-1.21 ms.
 constexpr int kRankThreads = 128;
-constexpr int kRankCap = 2048;  // keys of one shared-memory tile (24 KB with their segment words)
-
-// cells per block of k_cell_rank: a power of two giving about 1,280 keys per block at the
-// mean occupancy (so a tile rarely needs splitting)
-inline int rank_cells_per_block(int64_t n, int Nc) {
-    const double mean = Nc > 0 ? (double)n / (double)Nc : 1.0;
-    int cells = 1;
-    while (cells < 4096 && (double)(2 * cells) * mean <= 1280.0) cells *= 2;
-    return cells;
-}
+constexpr int kRankWarpCells = 8;  // consecutive cells of a warp, four at a time
+constexpr int kRankCells = kRankThreads / 32 * kRankWarpCells;  // cells per block
+constexpr int kRankGroupMax = 32;                               // entries of a cell ranked by eight lanes
+constexpr int kRankRow = kRankGroupMax + 4;  // ids of a group (four banks on from the last group's)
 
 __device__ __forceinline__ int seg_lo(uint64_t s) { return (int)(uint32_t)s; }
 
-// slots[start[c] + rank] = slot of the key of that rank among cell c's keys (ascending
-// particle id; ids are unique, so they alone rank a cell's keys). A block takes cellsPerBlock
-// consecutive cells, stages their ids and slots in shared memory (splitting the run of cells
-// where it exceeds kRankCap keys) and ranks each key against its own cell's ids. A cell above
-// kRankCap keys on its own is ranked from global memory.
-__device__ __forceinline__ void cell_rank_block(int blk, const uint64_t* __restrict__ start, int Nc, int cellsPerBlock,
+__device__ __forceinline__ int below4(uint4 q, uint32_t id) {
+    return (int)(q.x < id) + (int)(q.y < id) + (int)(q.z < id) + (int)(q.w < id);
+}
+
+// Cells [c0, c0 + kRankWarpCells) of a warp by groups of eight lanes, a cell each: a lane holds K of the cell's
+// keys (8K >= its entries m), and the group's ids lie padded with the largest id in row `sh`.
+// st: lane l <= kRankWarpCells holds the start of cell c0 + l. Cells above 8K entries are left out.
+template <int K>
+__device__ __forceinline__ void rank_groups(int st, const uint64_t* __restrict__ keys, int* __restrict__ slots,
+                                            uint32_t* sh) {
+    constexpr int kRounds = kRankWarpCells / 4;
+    const int lane = threadIdx.x & 31, k = lane & 7, g = lane >> 3;
+    int a[kRounds], m[kRounds];
+    uint64_t key[kRounds][K];
+#pragma unroll
+    for (int q = 0; q < kRounds; ++q) {
+        a[q] = __shfl_sync(0xffffffffu, st, 4 * q + g);
+        m[q] = __shfl_sync(0xffffffffu, st, 4 * q + g + 1) - a[q];
+        if (m[q] > 8 * K) m[q] = 0;
+#pragma unroll
+        for (int u = 0; u < K; ++u) key[q][u] = k + 8 * u < m[q] ? keys[a[q] + k + 8 * u] : ~0ULL;
+    }
+#pragma unroll
+    for (int q = 0; q < kRounds; ++q) {
+        uint32_t id[K];
+        int r[K];
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            id[u] = (uint32_t)(key[q][u] >> 32);
+            r[u] = 0;
+            sh[g * kRankRow + k + 8 * u] = id[u];
+        }
+        __syncwarp();
+        const int e = __reduce_max_sync(0xffffffffu, m[q]);
+#pragma unroll
+        for (int j = 0; j < 8 * K; j += 4) {
+            if (j >= e) break;
+            const uint4 w = *reinterpret_cast<const uint4*>(sh + g * kRankRow + j);
+#pragma unroll
+            for (int u = 0; u < K; ++u) r[u] += below4(w, id[u]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < K; ++u)
+            if (k + 8 * u < m[q]) slots[a[q] + r[u]] = (int)(uint32_t)key[q][u];
+    }
+}
+
+// A cell of m entries from a by a whole warp: 128 keys in registers against 128 ids in sh at a time.
+__device__ __noinline__ static void rank_cell_warp(int a, int m, const uint64_t* __restrict__ keys, int* __restrict__ slots,
+                                                   uint32_t* sh) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int i0 = 0; i0 < m; i0 += 128) {
+        uint64_t key[4];
+        int r[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) key[u] = i0 + lane + 32 * u < m ? keys[a + i0 + lane + 32 * u] : ~0ULL;
+#pragma unroll 1
+        for (int j0 = 0; j0 < m; j0 += 128) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                sh[lane + 32 * u] = j0 + lane + 32 * u < m ? (uint32_t)(keys[a + j0 + lane + 32 * u] >> 32) : 0xffffffffu;
+            __syncwarp();
+            const int e = min(128, m - j0);
+            for (int j = 0; j < e; j += 4) {
+                const uint4 w = *reinterpret_cast<const uint4*>(sh + j);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) r[u] += below4(w, (uint32_t)(key[u] >> 32));
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i0 + lane + 32 * u < m) slots[a + r[u]] = (int)(uint32_t)key[u];
+    }
+}
+
+// slots[start[c] + rank] = slot of the key of that rank among cell c's keys (ascending particle id;
+// ids are unique, so they alone rank a cell's keys, and none is the padding's 0xffffffff).
+__device__ __forceinline__ void cell_rank_block(int blk, const uint64_t* __restrict__ start, int Nc,
                                                 const uint64_t* __restrict__ keys, int* __restrict__ slots) {
-    __shared__ uint32_t kid[kRankCap];   // particle id
-    __shared__ int ksl[kRankCap];        // slot
-    __shared__ uint32_t seg[kRankCap];   // per key: its cell's segment [a, b) in the tile, a | b << 16
-    const int t = threadIdx.x;
-    const int c0 = (int)min((int64_t)blk * cellsPerBlock, (int64_t)Nc);
-    const int c1 = min(Nc, c0 + cellsPerBlock);
-    int cs = c0;
-    while (cs < c1) {  // block-uniform
-        const int A = seg_lo(start[cs]);
-        int ce = c1;
-        if (seg_lo(start[c1]) - A > kRankCap) {
-            int lo = cs, hi = c1 - 1;  // the last ce with start[ce] - A <= kRankCap
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (seg_lo(start[mid]) - A <= kRankCap)
-                    lo = mid;
-                else
-                    hi = mid - 1;
-            }
-            ce = lo;
-        }
-        if (ce == cs) {
-            const int b = seg_lo(start[cs + 1]);
-            for (int i = A + t; i < b; i += kRankThreads) {
-                const uint64_t k = keys[i];
-                const uint32_t id = (uint32_t)(k >> 32);
-                int r = 0;
-                for (int j = A; j < b; ++j) r += (uint32_t)(keys[j] >> 32) < id;
-                slots[A + r] = (int)(uint32_t)k;
-            }
-            ++cs;
-            continue;
-        }
-        const int m = seg_lo(start[ce]) - A;
-#pragma unroll 4
-        for (int i = t; i < m; i += kRankThreads) {
-            const uint64_t k = keys[A + i];
-            kid[i] = (uint32_t)(k >> 32);
-            ksl[i] = (int)(uint32_t)k;
-        }
-        for (int c = cs + t; c < ce; c += kRankThreads) {
-            const int a = seg_lo(start[c]) - A, b = seg_lo(start[c + 1]) - A;
-            for (int j = a; j < b; ++j) seg[j] = (uint32_t)a | ((uint32_t)b << 16);
-        }
-        __syncthreads();
-        for (int i = t; i < m; i += kRankThreads) {
-            const uint32_t sg = seg[i];
-            const int a = (int)(sg & 0xffffu), b = (int)(sg >> 16);
-            const uint32_t id = kid[i];
-            int r = 0;
-#pragma unroll 4
-            for (int j = a; j < b; ++j) r += kid[j] < id;
-            slots[A + a + r] = ksl[i];
-        }
-        __syncthreads();
-        cs = ce;
+    static_assert(4 * kRankRow >= 128 && kRankWarpCells < 32, "a warp's row of 128 ids; its starts in one load");
+    __shared__ __align__(16) uint32_t ids[kRankThreads / 32][4 * kRankRow];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    uint32_t* sh = ids[wib];
+    const int64_t c0 = (int64_t)blk * kRankCells + wib * kRankWarpCells;
+    if (c0 >= Nc) return;  // the whole warp; no block barrier follows
+    const int st = seg_lo(start[min(c0 + min(lane, kRankWarpCells), (int64_t)Nc)]);
+    const int m = __shfl_down_sync(0xffffffffu, st, 1) - st;  // 0 past the warp's cells
+    const int most = __reduce_max_sync(0xffffffffu, lane < kRankWarpCells && m <= kRankGroupMax ? m : 0);
+    if (most <= 16)
+        rank_groups<2>(st, keys, slots, sh);
+    else if (most <= 24)
+        rank_groups<3>(st, keys, slots, sh);
+    else
+        rank_groups<4>(st, keys, slots, sh);
+    for (unsigned big = __ballot_sync(0xffffffffu, lane < kRankWarpCells && m > kRankGroupMax); big; big &= big - 1) {
+        const int l = __ffs(big) - 1;
+        rank_cell_warp(__shfl_sync(0xffffffffu, st, l), __shfl_sync(0xffffffffu, m, l), keys, slots, sh);
     }
 }
 
 __global__ void __launch_bounds__(kRankThreads) k_cell_rank(const uint64_t* __restrict__ start, int Nc,
-                                                            int cellsPerBlock, const uint64_t* __restrict__ keys,
-                                                            int* __restrict__ slots) {
-    cell_rank_block((int)blockIdx.x, start, Nc, cellsPerBlock, keys, slots);
+                                                            const uint64_t* __restrict__ keys, int* __restrict__ slots) {
+    cell_rank_block((int)blockIdx.x, start, Nc, keys, slots);
 }
 
 // ------------------------------------------------------------------ batched index builds
@@ -356,7 +394,7 @@ struct IndexJob {
     int* slots;
     const int* pid;
     uint64_t* keys;
-    int n, Nc, rankCells;
+    int n, Nc;
 };
 
 // the job r with offs[r] <= b < offs[r + 1] (offs ascending, offs[0] = 0)
@@ -395,14 +433,14 @@ __global__ void k_scatter_keys_batch(const IndexJob* __restrict__ jobs, const in
     scatter_keys_block(b - offs[r], J.cid, J.pos, J.pid, J.n, J.start, J.keys);
 }
 
-// offs: blocks of each job's rank sort (ceil(Nc / rankCells))
+// offs: blocks of each job's rank sort (kRankCells cells per block)
 __global__ void __launch_bounds__(kRankThreads) k_cell_rank_batch(const IndexJob* __restrict__ jobs,
                                                                   const int* __restrict__ offs, int nJobs) {
     const int b = (int)blockIdx.x;
     if (nJobs <= 0 || b >= offs[nJobs]) return;
     const int r = job_of(offs, nJobs, b);
     const IndexJob J = jobs[r];
-    cell_rank_block(b - offs[r], J.start, J.Nc, J.rankCells, J.keys, J.slots);
+    cell_rank_block(b - offs[r], J.start, J.Nc, J.keys, J.slots);
 }
 
 }  // namespace mpcd_dev

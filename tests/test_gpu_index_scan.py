@@ -35,3 +35,29 @@ def test_sums_in_id_order(Nx, Ny):
     assert np.array_equal(f["N"], np.bincount(cid, minlength=Nx * Ny))
     assert np.array_equal(f["Px"], np.bincount(cid, weights=v[0::2], minlength=Nx * Ny))
     assert np.array_equal(f["Py"], np.bincount(cid, weights=v[1::2], minlength=Nx * Ny))
+
+
+# entries per cell around the rank sort's group sizes (8, 16, 24 and 32 entries, 128 keys of a warp),
+# in neighbouring cells and far apart
+COUNTS = [0, 1, 7, 8, 9, 15, 16, 17, 23, 24, 25, 31, 32, 33, 63, 64, 65, 127, 128, 129, 257, 700]
+
+
+@pytest.mark.parametrize("spread", [1, 5, 11])
+def test_order_within_cells(spread):
+    native = _native()
+    Nx, Ny = 23, 13
+    counts = np.zeros(Nx * Ny, np.int64)
+    counts[(np.arange(len(COUNTS)) * spread + 2) % (Nx * Ny)] = COUNTS
+    rng = np.random.default_rng(spread)
+    cid = rng.permutation(np.repeat(np.arange(Nx * Ny), counts))
+    p = poiseuille_params(Nx, Ny, 10, n=len(cid))
+    x = np.empty(2 * len(cid))
+    x[0::2] = (cid // Ny + rng.uniform(0.01, 0.99, len(cid))) * (p["Lx"] / Nx)
+    x[1::2] = (cid % Ny + rng.uniform(0.01, 0.99, len(cid))) * (p["Ly"] / Ny)
+    v = rng.standard_normal(2 * len(cid)) * 10.0 ** rng.integers(-6, 7, len(cid)).repeat(2)  # sums depend on the order
+    with native.Context(p) as ctx:
+        ctx.set_state(x, v)
+        f = ctx.cell_fields(3.0)
+    assert np.array_equal(f["N"], counts)
+    assert np.array_equal(f["Px"], np.bincount(cid, weights=v[0::2], minlength=Nx * Ny))
+    assert np.array_equal(f["Py"], np.bincount(cid, weights=v[1::2], minlength=Nx * Ny))
