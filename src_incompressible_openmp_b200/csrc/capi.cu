@@ -144,7 +144,7 @@ struct mpcd_ctx {
     cudaEvent_t bcDone = nullptr, wallsDone = nullptr;
     bool wallsPending = false;
     // CUDA-graph replay of the plain step: the step number and its seeds live on the device
-    // (step_begin, in k_srd_shift); one graph per entry parity of the ping-pong buffers
+    // (step_begin, in k_step_head); one graph per entry parity of the ping-pong buffers
     bool graphMode = false;            // true while a step is being captured
     bool useGraphs = true;
     long long* dStep = nullptr;        // device: number of the last step begun
@@ -2494,8 +2494,8 @@ static int step_once(mpcd_ctx* c, int64_t step, bool metrics, Prof* pf = nullptr
 
 // A step replayed from a CUDA graph. The graph of each entry parity of the ping-pong
 // buffers is captured from step_once on first use; the step number and seeds come from the
-// device (step_begin, run by the step's k_srd_shift, increments *dStep), so one graph serves every step. Needs the step's
-// sign stream prefetched by the step before (signsStep), like the eager path's fast case.
+// device (step_begin, run by the step's k_step_head, increments *dStep), so one graph serves every
+// step. Needs the step's sign stream prefetched by the step before (signsStep), like the eager path's fast case.
 static int graph_step(mpcd_ctx* c, int64_t step) {
     const int key = (c->xv * 2 + c->pp) * 2 + c->xflip;
     if (!c->gexec[key]) {

@@ -107,7 +107,7 @@ __device__ __forceinline__ void for_velocities(const V& S, const int* __restrict
 // The red state of a step whose shifted pass ran in place: `start` and `slots` are still the pass's
 // input index, and the few particles that changed cells are listed per new cell, with a flag per old
 // cell (ZoneArgs::arrHead ...). arrHead nullptr: the index is the red state's own. The lists and flags
-// are cleared as they are read. (An index rebuilt for at most a few moves per zone took 1.24 ms at
+// are cleared as they are read. (An index rebuilt for at most a few moves per zone takes 1.07 ms at
 // 84 M particles, the copy of the velocities for an out-of-place pass 0.40 ms.)
 struct RedPatch {
     int* arrHead;
