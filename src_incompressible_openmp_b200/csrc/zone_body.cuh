@@ -472,27 +472,7 @@ struct ZoneState {
     __device__ __forceinline__ double map_val(int l, bool low) const { return low ? map_low(l) : map_high(l); }
 
     // ------------------------------------------------------------------ smoothing, maps
-    // (Where the zone and its two-cell ring lie inside the domain, all nine weights apply and sum
-    // to 1: sixteenths of integers, exact in any order. The current counts go into the window, whose
-    // inner part nothing else reads.)
     __device__ void compute_nsm() {
-        if (fast && xs >= 2 && ys >= 2 && xe + 2 <= P().Nx && ye + 2 <= P().Ny) {
-            for (int l = lane; l < nl; l += kWarp) {
-                const int lx = lx_of(l);
-                M.win[(lx + 2) * WY + (l - lx * TY) + 2] = (typename ZoneMem<I>::W)M.len[l];
-            }
-            __syncwarp();
-            const int GY = TY + 2, G = (TX + 2) * GY;
-            const unsigned long long gyMagic = (unsigned long long)(0xffffffffu / (unsigned)GY) + 1ULL;  // as tyMagic
-            for (int g = lane; g < G; g += kWarp) {
-                const int gx = (int)(((unsigned long long)(unsigned)g * gyMagic) >> 32), gy = g - gx * GY;
-                const auto* w = M.win + (gx + 1) * WY + gy + 1;
-                const int s = w[-WY - 1] + w[-WY + 1] + w[WY - 1] + w[WY + 1] + 2 * (w[-WY] + w[WY] + w[-1] + w[1]) + 4 * w[0];
-                M.nsm[g] = (double)s * 0.0625;
-            }
-            __syncwarp();
-            return;
-        }
         zone_compute_nsm(M.nsm, M.win, M.len, xs, ys, TX, TY, P().Nx, P().Ny, P().perx, P().pery, lane);
     }
 
