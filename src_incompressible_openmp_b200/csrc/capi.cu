@@ -114,6 +114,7 @@ struct mpcd_ctx {
     bool srdCellsValid = false;
     CellIndex idxStd, idxSrd;
     bool idxStdValid = false;
+    bool stdOrderKept = false;     // not valid, but idxStd.slots is nearly the order of the next build
     // The step's shifted pass in place (ZoneArgs::corrSlot): few of its zones change anything, so the
     // corrected velocities are listed and, in plain steps (shiftPatched), so are the moved particles,
     // with which the closure reads the pass's input index instead of a new one. Off in a batch that
@@ -655,15 +656,18 @@ int scan_u64(mpcd_ctx* c, const uint64_t* in, int64_t n, uint64_t* out, cudaStre
 
 // I.count is all zero between builds (set at creation, cleared again by the scan's read).
 // s, keys, sums: the stream and scratch buffers (default: the context's stream, sortKeys and
-// blockSums).
+// blockSums). order: null, or a permutation of the slots to go through them by (slot_of_entry; may be
+// I.slots, which is written last).
 int build_index(mpcd_ctx* c, const int* cid, CellIndex& I, Prof* pf = nullptr, int label = -1,
-                cudaStream_t s = nullptr, uint64_t* keys = nullptr, uint64_t* sums = nullptr) {
+                cudaStream_t s = nullptr, uint64_t* keys = nullptr, uint64_t* sums = nullptr,
+                const int* order = nullptr) {
     if (!s) s = c->stream;
     if (!keys) keys = c->sortKeys;
     if (!sums) sums = c->blockSums;
     if (&I == &c->idxStd) c->idxIota = false;
     if (c->n > 0) {
-        k_histogram<<<blocks_for(c->n, kThreads * kIndexItems), kThreads, 0, s>>>(cid, c->n, I.count, I.pos);
+        auto* hist = order ? k_histogram<true> : k_histogram<false>;
+        hist<<<blocks_for(c->n, kThreads * kIndexItems), kThreads, 0, s>>>(cid, c->n, I.count, I.pos, order);
         ++c->launches;
     }
     if (c->Nc <= kSmallScan) {
@@ -676,8 +680,9 @@ int build_index(mpcd_ctx* c, const int* cid, CellIndex& I, Prof* pf = nullptr, i
         k_count_scan_apply<<<nb, kScanThreads, 0, s>>>(I.count, c->Nc, sums, I.start); ++c->launches;
     }
     if (c->n > 0) {
-        k_scatter_keys<<<blocks_for(c->n, kThreads * kIndexItems), kThreads, 0, s>>>(
-            cid, I.pos, c->pidb[c->pp], c->n, I.start, keys); ++c->launches;
+        auto* scatter = order ? k_scatter_keys<true> : k_scatter_keys<false>;
+        scatter<<<blocks_for(c->n, kThreads * kIndexItems), kThreads, 0, s>>>(cid, I.pos, c->pidb[c->pp], c->n, I.start,
+                                                                              keys, order); ++c->launches;
         k_cell_rank<<<blocks_for(c->Nc, kRankCells), kRankThreads, 0, s>>>(I.start, c->Nc, keys,
                                                                             I.slots); ++c->launches;
     }
@@ -756,7 +761,9 @@ int ensure_std_index(mpcd_ctx* c, Prof* pf = nullptr) {
         ++c->launches;
         c->cidStdValid = true;
     }
-    const int rc = build_index(c, c->cidStd, c->idxStd, pf, 5);
+    const int* order = c->stdOrderKept ? c->idxStd.slots : nullptr;
+    const int rc = build_index(c, c->cidStd, c->idxStd, pf, 5, nullptr, nullptr, nullptr, order);
+    c->stdOrderKept = false;
     if (!rc) c->idxStdValid = true;
     return rc;
 }
@@ -765,6 +772,7 @@ void invalidate_positions(mpcd_ctx* c) {
     c->cidStdValid = false;
     c->idxStdValid = false;
     c->srdCellsValid = false;
+    c->stdOrderKept = false;
 }
 
 // ---------------------------------------------------------------- host <-> device in id order
@@ -1205,6 +1213,7 @@ void zone_pass_flip(mpcd_ctx* c) {
     // cid was updated for moved particles; positions changed. A patched pass leaves its input's index
     // to the closure.
     c->idxStdValid = c->zA.moverSlot != nullptr;
+    c->stdOrderKept = !c->idxStdValid;
     c->srdCellsValid = false;
 }
 
@@ -2398,7 +2407,7 @@ static int step_head(mpcd_ctx* c, int64_t step, bool metrics, Prof* pf) {
     if (rc) return rc;
     c->cidStdValid = true;
     c->srdCellsValid = true;
-    c->idxStdValid = false;
+    c->idxStdValid = c->stdOrderKept = false;
     if (overlap) {
         // the standard-grid index on the walls stream, after the wall kernels (whose end the
         // collision waits for), beside the SRD index and the collision on the main stream
@@ -3133,7 +3142,7 @@ static int batch_index(mpcd_batch* b) {
     CUDA_TRY(cudaGetLastError());
     for (mpcd_ctx* c : b->members) {
         c->idxStdValid = true;
-        c->idxIota = false;
+        c->idxIota = c->stdOrderKept = false;
     }
     return MPCD_OK;
 }
@@ -3380,7 +3389,7 @@ int mpcd_batch_create(const mpcd_params_c* params, int count, int device, mpcd_b
             for (mpcd_ctx* c : b->members) {
                 CellIndex& I = c->idxStd;
                 jobs.push_back(IndexJob{c->cidStd, I.count, I.pos, I.start, I.slots, c->pidb[q], c->sortKeys, c->n,
-                                        c->Nc});
+                                        c->Nc, nullptr});
             }
             ok = cudaMalloc((void**)&b->dJobs[q], sizeof(IndexJob) * jobs.size()) == cudaSuccess &&
                  cudaMemcpy(b->dJobs[q], jobs.data(), sizeof(IndexJob) * jobs.size(), cudaMemcpyHostToDevice) ==

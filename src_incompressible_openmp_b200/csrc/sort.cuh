@@ -200,13 +200,25 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_counts_small(int* __restr
 // covers kIndexItems runs of 32 consecutive slots, whose atomics are in flight together.
 constexpr int kIndexItems = 4;
 
+// The slots in the order of an earlier index: `order`, a permutation of them all, when kOrder. Few
+// particles change cells between the two builds around a base pass, so consecutive entries form
+// runs of whole cells there, where consecutive slots (ordered by the cells before the streaming) hold
+// runs of one or two. pos is by entry then.
+template <bool kOrder>
+__device__ __forceinline__ int slot_of_entry(const int* __restrict__ order, int j) {
+    return kOrder ? order[j] : j;
+}
+
+template <bool kOrder>
 __device__ __forceinline__ void histogram_block(int blk, const int* __restrict__ cid, int n, int* __restrict__ count,
-                                                int* __restrict__ pos) {
+                                                int* __restrict__ pos, const int* __restrict__ order) {
     const int lane = threadIdx.x & 31;
     const int base = ((blk * (int)blockDim.x + (int)threadIdx.x) >> 5) * (32 * kIndexItems) + lane;
     int c[kIndexItems], got[kIndexItems], runStart[kIndexItems];
 #pragma unroll
-    for (int k = 0; k < kIndexItems; ++k) c[k] = (base + 32 * k < n) ? cid[base + 32 * k] : -1;
+    for (int k = 0; k < kIndexItems; ++k) c[k] = (base + 32 * k < n) ? slot_of_entry<kOrder>(order, base + 32 * k) : -1;
+#pragma unroll
+    for (int k = 0; k < kIndexItems; ++k) c[k] = c[k] >= 0 ? cid[c[k]] : -1;
 #pragma unroll
     for (int k = 0; k < kIndexItems; ++k) {
         const int prev = __shfl_up_sync(0xffffffffu, c[k], 1);
@@ -225,38 +237,44 @@ __device__ __forceinline__ void histogram_block(int blk, const int* __restrict__
     }
 }
 
-__global__ void k_histogram(const int* __restrict__ cid, int n, int* __restrict__ count, int* __restrict__ pos) {
-    histogram_block((int)blockIdx.x, cid, n, count, pos);
+template <bool kOrder>
+__global__ void k_histogram(const int* __restrict__ cid, int n, int* __restrict__ count, int* __restrict__ pos,
+                            const int* __restrict__ order) {
+    histogram_block<kOrder>((int)blockIdx.x, cid, n, count, pos, order);
 }
 
 // keys[start[cid[s]] + pos[s]] = (pid[s] << 32) | s: each cell's segment holds its
-// particles' keys in arrival order (same slot coverage as k_histogram)
+// particles' keys in arrival order (same slot coverage and order as k_histogram)
+template <bool kOrder>
 __device__ __forceinline__ void scatter_keys_block(int blk, const int* __restrict__ cid, const int* __restrict__ pos,
                                                    const int* __restrict__ pid, int n,
-                                                   const uint64_t* __restrict__ start, uint64_t* __restrict__ keys) {
+                                                   const uint64_t* __restrict__ start, uint64_t* __restrict__ keys,
+                                                   const int* __restrict__ order) {
     const int lane = threadIdx.x & 31;
     const int base = ((blk * (int)blockDim.x + (int)threadIdx.x) >> 5) * (32 * kIndexItems) + lane;
-    int c[kIndexItems], p[kIndexItems], q[kIndexItems];
+    int t[kIndexItems], c[kIndexItems], p[kIndexItems], q[kIndexItems];
+#pragma unroll
+    for (int k = 0; k < kIndexItems; ++k) t[k] = base + 32 * k < n ? slot_of_entry<kOrder>(order, base + 32 * k) : -1;
 #pragma unroll
     for (int k = 0; k < kIndexItems; ++k) {
-        const int s = base + 32 * k;
-        c[k] = s < n ? cid[s] : 0;
-        p[k] = s < n ? pos[s] : 0;
-        q[k] = s < n ? pid[s] : 0;
+        c[k] = t[k] >= 0 ? cid[t[k]] : 0;
+        p[k] = t[k] >= 0 ? pos[base + 32 * k] : 0;
+        q[k] = t[k] >= 0 ? pid[t[k]] : 0;
     }
     uint32_t at[kIndexItems];
 #pragma unroll
     for (int k = 0; k < kIndexItems; ++k) at[k] = (uint32_t)start[c[k]];
 #pragma unroll
     for (int k = 0; k < kIndexItems; ++k) {
-        const int s = base + 32 * k;
-        if (s < n) keys[at[k] + p[k]] = ((uint64_t)(uint32_t)q[k] << 32) | (uint32_t)s;
+        if (t[k] >= 0) keys[at[k] + p[k]] = ((uint64_t)(uint32_t)q[k] << 32) | (uint32_t)t[k];
     }
 }
 
+template <bool kOrder>
 __global__ void k_scatter_keys(const int* __restrict__ cid, const int* __restrict__ pos, const int* __restrict__ pid,
-                               int n, const uint64_t* __restrict__ start, uint64_t* __restrict__ keys) {
-    scatter_keys_block((int)blockIdx.x, cid, pos, pid, n, start, keys);
+                               int n, const uint64_t* __restrict__ start, uint64_t* __restrict__ keys,
+                               const int* __restrict__ order) {
+    scatter_keys_block<kOrder>((int)blockIdx.x, cid, pos, pid, n, start, keys, order);
 }
 
 // Rank sort of the cells' keys. Eight lanes take a cell of up to 32 entries: their keys stay in
@@ -395,6 +413,7 @@ struct IndexJob {
     const int* pid;
     uint64_t* keys;
     int n, Nc;
+    const int* order;  // nullable (slot_of_entry)
 };
 
 // the job r with offs[r] <= b < offs[r + 1] (offs ascending, offs[0] = 0)
@@ -416,7 +435,10 @@ __global__ void k_histogram_batch(const IndexJob* __restrict__ jobs, const int* 
     if (nJobs <= 0 || b >= offs[nJobs]) return;
     const int r = job_of(offs, nJobs, b);
     const IndexJob J = jobs[r];
-    histogram_block(b - offs[r], J.cid, J.n, J.count, J.pos);
+    if (J.order)
+        histogram_block<true>(b - offs[r], J.cid, J.n, J.count, J.pos, J.order);
+    else
+        histogram_block<false>(b - offs[r], J.cid, J.n, J.count, J.pos, nullptr);
 }
 
 // one block per job (every job has Nc <= kSmallScan)
@@ -430,7 +452,10 @@ __global__ void k_scatter_keys_batch(const IndexJob* __restrict__ jobs, const in
     if (nJobs <= 0 || b >= offs[nJobs]) return;
     const int r = job_of(offs, nJobs, b);
     const IndexJob J = jobs[r];
-    scatter_keys_block(b - offs[r], J.cid, J.pos, J.pid, J.n, J.start, J.keys);
+    if (J.order)
+        scatter_keys_block<true>(b - offs[r], J.cid, J.pos, J.pid, J.n, J.start, J.keys, J.order);
+    else
+        scatter_keys_block<false>(b - offs[r], J.cid, J.pos, J.pid, J.n, J.start, J.keys, nullptr);
 }
 
 // offs: blocks of each job's rank sort (kRankCells cells per block)
