@@ -3756,21 +3756,24 @@ int mpcd_learned_grad(const float* features, const float* targets, int64_t rows,
     int* dI;
     DevStatus* dS;
     int sms = 0;
-    if ((rc = D.open(device)) || (rc = D.alloc(&dX, (size_t)rows * kFeat)) || (rc = D.alloc(&dY, (size_t)rows * kOut)) ||
+    if ((rc = D.open(device)) || (rc = tg_setup(device, &sms))) return rc;
+    const int ctas = tg_grid((int)rows, sms);
+    // the CTAs' partial gradients lie behind the rows (an allocation of their own cost the call 0.5 ms)
+    if ((rc = D.alloc(&dX, (size_t)rows * kFeat + (size_t)ctas * kParams)) || (rc = D.alloc(&dY, (size_t)rows * kOut)) ||
         (rc = D.alloc(&dP, kParams)) || (rc = D.alloc(&dG, kParams)) || (rc = D.alloc(&dL, 1)) ||
-        (rc = D.alloc(&dI, (size_t)rows)) || (rc = D.alloc(&dS, 1)) || (rc = tg_setup(device, &sms)))
+        (rc = D.alloc(&dI, (size_t)rows)) || (rc = D.alloc(&dS, 1)))
         return rc;
+    float* dSlabs = dX + (size_t)rows * kFeat;
     std::vector<int> idx((size_t)rows);
     for (int64_t i = 0; i < rows; ++i) idx[(size_t)i] = (int)i;
     CUDA_TRY(cudaMemcpyAsync(dX, features, sizeof(float) * kFeat * rows, cudaMemcpyHostToDevice, D.stream));
     CUDA_TRY(cudaMemcpyAsync(dY, targets, sizeof(float) * kOut * rows, cudaMemcpyHostToDevice, D.stream));
     CUDA_TRY(cudaMemcpyAsync(dP, params, sizeof(float) * kParams, cudaMemcpyHostToDevice, D.stream));
     CUDA_TRY(cudaMemcpyAsync(dI, idx.data(), sizeof(int) * rows, cudaMemcpyHostToDevice, D.stream));
-    CUDA_TRY(cudaMemsetAsync(dG, 0, sizeof(float) * kParams, D.stream));
-    CUDA_TRY(cudaMemsetAsync(dL, 0, sizeof(float), D.stream));
     CUDA_TRY(cudaMemsetAsync(dS, 0, sizeof(DevStatus), D.stream));
-    k_mlp_grad_tc<<<tg_grid((int)rows, sms), kTgThreads, kTgSmem, D.stream>>>(dX, dY, dI, (int)rows, (int)rows,
-                                                                       1.0f / params[kOffScale], dP, dG, dL, dS);
+    k_mlp_grad_tc<<<ctas, kTgThreads, kTgSmem, D.stream>>>(dX, dY, dI, (int)rows, (int)rows, 1.0f / params[kOffScale], dP,
+                                                           dSlabs, dS);
+    k_grad_sum<<<(kParams + 255) / 256, 256, 0, D.stream>>>(dSlabs, ctas, dG, dL);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(grad, dG, sizeof(float) * kParams, cudaMemcpyDeviceToHost, D.stream));
     CUDA_TRY(cudaMemcpyAsync(loss, dL, sizeof(float), cudaMemcpyDeviceToHost, D.stream));
@@ -3790,21 +3793,24 @@ int mpcd_learned_train(const float* features, const float* targets, int64_t rows
         params[kOffScale] = (float)(rms > 0.0 ? rms : 1.0);
     }
     LearnedDev D;
-    float *dX, *dY, *dP, *dG, *dM, *dV, *dL;
+    float *dX, *dY, *dP, *dM, *dV, *dL;
     int* dI;
     DevStatus* dS;
     int sms = 0;
     const int64_t nb = (rows + batch - 1) / batch;
-    if ((rc = D.open(device)) || (rc = D.alloc(&dX, (size_t)rows * kFeat)) || (rc = D.alloc(&dY, (size_t)rows * kOut)) ||
-        (rc = D.alloc(&dP, kParams)) || (rc = D.alloc(&dG, kParams)) || (rc = D.alloc(&dM, kParams)) ||
+    if ((rc = D.open(device)) || (rc = tg_setup(device, &sms))) return rc;
+    const size_t slabs = (size_t)tg_grid((int)std::min<int64_t>(batch, rows), sms) * kParams;  // behind the rows
+    if ((rc = D.alloc(&dX, (size_t)rows * kFeat + slabs)) || (rc = D.alloc(&dY, (size_t)rows * kOut)) ||
+        (rc = D.alloc(&dP, kParams)) || (rc = D.alloc(&dM, kParams)) ||
         (rc = D.alloc(&dV, kParams)) || (rc = D.alloc(&dL, (size_t)nb)) || (rc = D.alloc(&dI, (size_t)rows)) ||
-        (rc = D.alloc(&dS, 1)) || (rc = tg_setup(device, &sms)))
+        (rc = D.alloc(&dS, 1)))
         return rc;
+    float* dSlabs = dX + (size_t)rows * kFeat;
     CUDA_TRY(cudaMemsetAsync(dS, 0, sizeof(DevStatus), D.stream));
     CUDA_TRY(cudaMemcpyAsync(dX, features, sizeof(float) * kFeat * rows, cudaMemcpyHostToDevice, D.stream));
     CUDA_TRY(cudaMemcpyAsync(dY, targets, sizeof(float) * kOut * rows, cudaMemcpyHostToDevice, D.stream));
     CUDA_TRY(cudaMemcpyAsync(dP, params, sizeof(float) * kParams, cudaMemcpyHostToDevice, D.stream));
-    for (float* b : {dG, dM, dV}) CUDA_TRY(cudaMemsetAsync(b, 0, sizeof(float) * kParams, D.stream));
+    for (float* b : {dM, dV}) CUDA_TRY(cudaMemsetAsync(b, 0, sizeof(float) * kParams, D.stream));
     const float yinv = 1.0f / params[kOffScale];
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     std::vector<int> idx((size_t)rows);
@@ -3816,15 +3822,15 @@ int mpcd_learned_train(const float* features, const float* targets, int64_t rows
         for (int64_t i = rows - 1; i > 0; --i) std::swap(idx[(size_t)i], idx[(size_t)(rng() % (uint64_t)(i + 1))]);
         CUDA_TRY(cudaStreamSynchronize(D.stream));  // idx is re-filled on the host
         CUDA_TRY(cudaMemcpyAsync(dI, idx.data(), sizeof(int) * rows, cudaMemcpyHostToDevice, D.stream));
-        CUDA_TRY(cudaMemsetAsync(dL, 0, sizeof(float) * nb, D.stream));
         for (int64_t b = 0; b < nb; ++b) {
             const int64_t r0 = b * batch;
             const int n = (int)std::min<int64_t>(batch, rows - r0);
             ++t;
-            k_mlp_grad_tc<<<tg_grid(n, sms), kTgThreads, kTgSmem, D.stream>>>(dX, dY, dI + r0, n, n, yinv, dP, dG, dL + b, dS);
-            k_adam<<<(kTrained + 255) / 256, 256, 0, D.stream>>>(dP, dG, dM, dV, kTrained, lr, b1, b2, eps,
-                                                                 1.0f - (float)std::pow((double)b1, (double)t),
-                                                                 1.0f - (float)std::pow((double)b2, (double)t));
+            const int ctas = tg_grid(n, sms);
+            k_mlp_grad_tc<<<ctas, kTgThreads, kTgSmem, D.stream>>>(dX, dY, dI + r0, n, n, yinv, dP, dSlabs, dS);
+            k_adam<<<(kParams + 255) / 256, 256, 0, D.stream>>>(dP, dSlabs, ctas, dM, dV, lr, b1, b2, eps,
+                                                                1.0f - (float)std::pow((double)b1, (double)t),
+                                                                1.0f - (float)std::pow((double)b2, (double)t), dL + b);
         }
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaMemcpyAsync(lossB.data(), dL, sizeof(float) * nb, cudaMemcpyDeviceToHost, D.stream));

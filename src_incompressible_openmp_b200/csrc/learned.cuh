@@ -226,18 +226,58 @@ __global__ void k_learned_samples(DevParams P, const float4* __restrict__ feat, 
     Y[2 * (size_t)s + 1] = (float)__dadd_rn(__dmul_rn(beta, duRY[c]), eosY[c]);
 }
 
-// Adam (Kingma & Ba) on the FP32 master weights; clears the gradient for the next batch.
-__global__ void k_adam(float* __restrict__ params, float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v,
-                       int count, float lr, float b1, float b2, float eps, float c1, float c2) {
+// Entry i of the sum of the n CTAs' partial gradients (k_mlp_grad_tc: rows of kParams). The order is fixed,
+// so a gradient, and a network trained with it, is the same in every run: FP32 sums depend on their order,
+// and a last bit that crosses a BF16 rounding boundary moves a network by up to 4e-5 within 64 Adam steps.
+// CTAs 4, 5, .. come first, then 2, 3, then 0, 1: the order in which FP32 atomics of one-tile CTAs mostly
+// arrive (four and eight tiles), so that networks trained with such atomics are met to 3e-8.
+__device__ __forceinline__ float grad_sum(const float* __restrict__ slabs, int n, int i) {
+    const float* p = slabs + i;
+    float h[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) h[q] = q < n ? p[q * kParams] : 0.0f;
+    float a = 0.0f;
+    for (int q0 = 4; q0 < n; q0 += 24) {  // 24 loads in flight
+        float w[24];
+#pragma unroll
+        for (int u = 0; u < 24; ++u) w[u] = q0 + u < n ? p[(size_t)(q0 + u) * kParams] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < 24; ++u)
+            if (q0 + u < n) a += w[u];
+    }
+    if (n > 2) a += h[2];
+    if (n > 3) a += h[3];
+    a += h[0];
+    if (n > 1) a += h[1];
+    return a;
+}
+
+// the summed gradient and loss of n CTAs
+__global__ void k_grad_sum(const float* __restrict__ slabs, int n, float* __restrict__ grad, float* __restrict__ loss) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const float g = grad[i];
+    if (i < kTrained) grad[i] = grad_sum(slabs, n, i);
+    if (i == kTrained) {
+        grad[i] = 0.0f;  // the output scale is not trained
+        *loss = grad_sum(slabs, n, i);
+    }
+}
+
+// Adam (Kingma & Ba) on the FP32 master weights from n CTAs' partial gradients; the batch's loss.
+__global__ void k_adam(float* __restrict__ params, const float* __restrict__ slabs, int n, float* __restrict__ m,
+                       float* __restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2,
+                       float* __restrict__ loss) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > kTrained) return;
+    const float g = grad_sum(slabs, n, i);
+    if (i == kTrained) {
+        *loss = g;
+        return;
+    }
     const float mi = b1 * m[i] + (1.0f - b1) * g;
     const float vi = b2 * v[i] + (1.0f - b2) * g * g;
     m[i] = mi;
     v[i] = vi;
     params[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    grad[i] = 0.0f;
 }
 
 // ---------------------------------------------------------------- tensor-core inference
@@ -622,9 +662,10 @@ __device__ __forceinline__ void tg_put(unsigned char* sm, uint32_t off, int r, i
 
 __global__ void __launch_bounds__(kTgThreads, 1)
     k_mlp_grad_tc(const float* __restrict__ X, const float* __restrict__ Y, const int* __restrict__ idx, int rows,
-                  int batch, float yinv, const float* __restrict__ params, float* __restrict__ grad,
-                  float* __restrict__ loss, DevStatus* st) {
+                  int batch, float yinv, const float* __restrict__ params, float* __restrict__ slabs, DevStatus* st) {
     extern __shared__ __align__(128) unsigned char sm[];
+    __shared__ float sLoss[4];
+    float* grad = slabs + (size_t)blockIdx.x * kParams;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int row = t & 127, g = t >> 7, h0 = 16 * g;  // this thread's row, warpgroup and first hidden unit
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
@@ -814,8 +855,8 @@ __global__ void __launch_bounds__(kTgThreads, 1)
         if (!sync_mma([&] { tg_mma(tmem + 4 * kHid, sbase + kTgOffXT, sbase + kTgOffD1T, kTgKR, !first); })) break;
         first = false;
     }
-    // the accumulated gradients: lane row of dW1^T is an operand column (feature, or b1 at 75), lane
-    // row of dW2^T an A1 column (or b2 at 64)
+    // the accumulated gradients, to this CTA's row of slabs (its loss in the scale's place): lane row of
+    // dW1^T is an operand column (feature, or b1 at 75), lane row of dW2^T an A1 column (or b2 at 64)
     if (ok && !first) {
         const int pk = row < kFeat ? (row % 3) * 25 + row / 3 : -1;
         uint32_t a[16], b[16];
@@ -826,22 +867,23 @@ __global__ void __launch_bounds__(kTgThreads, 1)
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
             const int j = h0 + q;
-            if (row < kFeat) atomicAdd(grad + kOffW1 + j * kFeat + pk, __uint_as_float(a[q]));
-            else if (row == kFeat) atomicAdd(grad + kOffB1 + j, __uint_as_float(a[q]));
-            if (row < kHid) atomicAdd(grad + kOffW2 + j * kHid + row, __uint_as_float(b[q]));
-            else if (row == kHid) atomicAdd(grad + kOffB2 + j, __uint_as_float(b[q]));
+            if (row < kFeat) grad[kOffW1 + j * kFeat + pk] = __uint_as_float(a[q]);
+            else if (row == kFeat) grad[kOffB1 + j] = __uint_as_float(a[q]);
+            if (row < kHid) grad[kOffW2 + j * kHid + row] = __uint_as_float(b[q]);
+            else if (row == kHid) grad[kOffB2 + j] = __uint_as_float(b[q]);
         }
         if (g == 0) {
-            atomicAdd(grad + kOffW3 + row, accW3);
-            if (row % kHid == 0) atomicAdd(grad + kOffB3 + row / kHid, accB3);
+            grad[kOffW3 + row] = accW3;
+            if (row % kHid == 0) grad[kOffB3 + row / kHid] = accB3;
         }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) lossAcc += __shfl_xor_sync(0xffffffffu, lossAcc, o);
-    if (lane == 0 && lossAcc != 0.0f) atomicAdd(loss, lossAcc);
+    if (lane == 0 && g == 0) sLoss[warp] = lossAcc;
     if (!ok) tc_wait(bar, phase ^ 1);  // an MMA did not complete in time: one more bounded wait
     tc_fence_before();
     __syncthreads();
+    if (t == 0) grad[kTrained] = ((sLoss[0] + sLoss[1]) + sLoss[2]) + sLoss[3];
     if (warp == 0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTgTmemCols) : "memory");
