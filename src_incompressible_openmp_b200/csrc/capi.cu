@@ -36,6 +36,13 @@
 
 using namespace mpcd_dev;
 
+// Device memory of the allocation helpers (dalloc, fb_upload): cudaMalloc, called through a pointer so
+// that tests can put a failing call in its place.
+static cudaError_t device_malloc(void** p, size_t bytes) { return cudaMalloc(p, bytes); }
+extern "C" {
+cudaError_t (*mpcd_device_malloc)(void**, size_t) = device_malloc;
+}
+
 namespace {
 
 thread_local std::string g_err;
@@ -434,7 +441,7 @@ template <typename T>
 int dalloc(T** p, size_t count) {
     *p = nullptr;
     if (count == 0) count = 1;
-    CUDA_TRY(cudaMalloc((void**)p, count * sizeof(T)));
+    CUDA_TRY(mpcd_device_malloc((void**)p, count * sizeof(T)));
     return MPCD_OK;
 }
 
@@ -3059,19 +3066,32 @@ struct mpcd_batch {
     int histBlocks = 0, rankBlocks = 0;
 };
 
+// the buffers of batch_status, made before a batch's first step (dStatus last: it stands for all three)
+static int batch_status_open(mpcd_batch* b) {
+    if (b->dStatus) return MPCD_OK;
+    const size_t n = b->members.size();
+    std::vector<DevStatus*> st;
+    for (mpcd_ctx* c : b->members) st.push_back(c->st);
+    if (!b->hCodes) CUDA_TRY(cudaMallocHost((void**)&b->hCodes, sizeof(int) * n));
+    DevStatus** d = nullptr;
+    int rc = b->dCodes ? MPCD_OK : dalloc(&b->dCodes, n);
+    if (!rc) rc = dalloc(&d, n);
+    if (!rc && cudaMemcpy(d, st.data(), sizeof(DevStatus*) * n, cudaMemcpyHostToDevice) != cudaSuccess) {
+        rc = set_err(MPCD_ERR_CUDA, "batch status table");
+        cudaFree(d);
+    }
+    if (rc) {
+        cudaGetLastError();
+        return rc;
+    }
+    b->dStatus = d;
+    return MPCD_OK;
+}
+
 // The device status of every member after a batched call, whose work is all on the batch stream: the
 // codes in one copy, then check_device of the first member that raised one.
 static int batch_status(mpcd_batch* b) {
     const int n = (int)b->members.size();
-    if (!b->dStatus) {
-        std::vector<DevStatus*> st;
-        for (mpcd_ctx* c : b->members) st.push_back(c->st);
-        CUDA_TRY(cudaMallocHost((void**)&b->hCodes, sizeof(int) * (size_t)n));
-        int rc = dalloc(&b->dCodes, (size_t)n);
-        if (!rc) rc = dalloc(&b->dStatus, (size_t)n);
-        if (rc) return rc;
-        CUDA_TRY(cudaMemcpy(b->dStatus, st.data(), sizeof(DevStatus*) * (size_t)n, cudaMemcpyHostToDevice));
-    }
     k_gather_status<<<(n + 255) / 256, 256, 0, b->stream>>>(b->dStatus, n, b->dCodes);
     ++b->members[0]->launches;
     CUDA_TRY(cudaGetLastError());
@@ -3457,9 +3477,16 @@ int mpcd_batch_step(mpcd_batch* b, int64_t step0, int64_t nsteps, double* device
     for (mpcd_ctx* c : b->members) together = together && f64_batch_takes(c);
     if (together) {
         for (mpcd_ctx* c : b->members) CUDA_TRY(cudaStreamSynchronize(c->stream));
-        CUDA_TRY(cudaEventRecord(b->start, b->stream));
-        const int rc = f64_batch_steps(b, step0, nsteps);
+        int rc = batch_status_open(b);
+        if (!rc) rc = f64_batch_open(b);
         if (rc) return rc;
+        CUDA_TRY(cudaEventRecord(b->start, b->stream));
+        rc = f64_batch_steps(b, step0, nsteps);
+        if (rc) {
+            // the members go on from the steps already launched, on their own streams
+            for (cudaStream_t q : {b->stream, b->f64->walls, b->f64->side}) cudaStreamSynchronize(q);
+            return rc;
+        }
         CUDA_TRY(cudaEventRecord(b->stop, b->stream));
         CUDA_TRY(cudaEventSynchronize(b->stop));
         float ms = 0.f;
