@@ -3105,11 +3105,20 @@ static int batch_status(mpcd_batch* b) {
 #include "fast_batch.inc"
 #include "f64_batch.inc"
 
+// The staging slot of a pass's arguments: by member 0's buffers, and apart for captured steps, whose
+// copies read their slot again at every replay. (Captured steps have every member's buffers lie alike;
+// eager ones fill the slots for members that may lie differently.)
+constexpr int kBatchSlots = 16;
+static int batch_slot(const mpcd_batch* b, int pass) {
+    const mpcd_ctx* c = b->members[0];
+    return (((c->graphMode ? 1 : 0) * 2 + (c->xv & 1)) * 2 + (c->xflip & 1)) * 2 + pass;
+}
+
 // the zone kernels of pass `pass` (0 base, 1 shifted) of every replica in one launch; each
 // replica's zone_pass_prep has filled its zA
 static int batch_zone_kernel(mpcd_batch* b, int pass) {
     const int n = (int)b->members.size();
-    const int slot = ((b->members[0]->xv & 1) * 2 + (b->members[0]->xflip & 1)) * 2 + pass;
+    const int slot = batch_slot(b, pass);
     ZoneArgs* h = b->hArgs + (size_t)slot * n;
     int* ho = b->hOffs + (size_t)slot * (n + 1);
     ho[0] = 0;
@@ -3171,7 +3180,7 @@ static int batch_index(mpcd_batch* b) {
 // the batched zone kernel), then each replica's host-side flip; staged like the zone arguments
 static int batch_zone_finish(mpcd_batch* b, int pass) {
     const int n = (int)b->members.size();
-    const int slot = ((b->members[0]->xv & 1) * 2 + (b->members[0]->xflip & 1)) * 2 + pass;
+    const int slot = batch_slot(b, pass);
     OverflowJob* h = b->hOv + (size_t)slot * n;
     for (int r = 0; r < n; ++r) h[r] = overflow_job(b->members[r], false);
     OverflowJob* d = b->dOv + (size_t)slot * n;
@@ -3354,9 +3363,9 @@ int mpcd_batch_create(const mpcd_params_c* params, int count, int device, mpcd_b
         return set_err(MPCD_ERR_CUDA, "batch stream");
     }
     {
-        // staging of the batched zone kernels (8 slots: velocity and position buffer x pass), the shared
-        // memory of the largest working set plus the arguments, the step counters
-        const size_t nslots = 8;
+        // staging of the batched zone kernels, the shared memory of the largest working set plus the
+        // arguments, the step counters
+        const size_t nslots = kBatchSlots;
         std::vector<long long*> steps((size_t)count);
         for (int r = 0; r < count; ++r) {
             b->zSmem = std::max(b->zSmem, b->members[r]->zSmem + (size_t)kZoneArgsSmem);
