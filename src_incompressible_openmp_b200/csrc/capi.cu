@@ -160,6 +160,7 @@ struct mpcd_ctx {
     cudaEvent_t sideDone = nullptr;    // the captured step joins its sign prefetch
     cudaGraphExec_t gexec[8] = {};  // by (xv, pp, xflip) at step entry
     int64_t gkernels[8] = {};
+    int64_t setup = 0;  // raised when an option changes that captured steps hold (drop_graphs)
     struct HostFlags {
         int xv, pp, xflip;
         bool cidStdValid, srdCellsValid, idxStdValid, idxIota, refValid;
@@ -2508,6 +2509,16 @@ static int step_once(mpcd_ctx* c, int64_t step, bool metrics, Prof* pf = nullptr
     return rc;
 }
 
+// captured steps (a batch's too) are made again after a change of what they hold
+static void drop_graphs(mpcd_ctx* c) {
+    ++c->setup;
+    for (auto& g : c->gexec)
+        if (g) {
+            cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
+}
+
 // A step replayed from a CUDA graph. The graph of each entry parity of the ping-pong
 // buffers is captured from step_once on first use; the step number and seeds come from the
 // device (step_begin, run by the step's k_step_head, increments *dStep), so one graph serves every
@@ -3054,6 +3065,7 @@ struct mpcd_batch {
     // whole batched steps replayed from CUDA graphs, one per buffer parity of the replicas
     bool useGraphs = true;
     cudaGraphExec_t gexec[8] = {};  // by (xv, pp, xflip) of the replicas at step entry
+    int64_t setup = 0;              // the members' setup counts when gexec was captured, summed
     std::vector<mpcd_ctx::HostFlags> gpost[8];
     std::vector<int64_t> gkernels[8];
     long long** dStepPtrs = nullptr;  // each replica's device step counter
@@ -3290,11 +3302,7 @@ int mpcd_ctx_collide_shape(mpcd_ctx* c, int32_t shape, int32_t* in_use) {
     if (shape >= 0) {
         CUDA_TRY(cudaSetDevice(c->device));
         CUDA_TRY(cudaStreamSynchronize(c->stream));
-        for (auto& g : c->gexec)  // captured steps hold the previous shape
-            if (g) {
-                cudaGraphExecDestroy(g);
-                g = nullptr;
-            }
+        drop_graphs(c);  // captured steps hold the previous shape
         c->collideShape = shape;
     }
     if (in_use) *in_use = c->collideShape;
@@ -3503,6 +3511,16 @@ int mpcd_batch_step(mpcd_batch* b, int64_t step0, int64_t nsteps, double* device
         if (device_seconds) *device_seconds = ms * 1e-3;
         return batch_status(b);
     }
+    int64_t setup = 0;
+    for (mpcd_ctx* c : b->members) setup += c->setup;
+    if (setup != b->setup) {  // a member's closure or collision shape changed
+        for (auto& g : b->gexec)
+            if (g) {
+                cudaGraphExecDestroy(g);
+                g = nullptr;
+            }
+        b->setup = setup;
+    }
     CUDA_TRY(cudaEventRecord(b->start, b->stream));
     for (mpcd_ctx* c : b->members) CUDA_TRY(cudaStreamWaitEvent(c->stream, b->start, 0));
     for (int64_t k = 1; k <= nsteps; ++k) {
@@ -3537,14 +3555,6 @@ int mpcd_batch_step(mpcd_batch* b, int64_t step0, int64_t nsteps, double* device
 }  // extern "C"
 
 // ---------------------------------------------------------------- learned closure
-static void drop_graphs(mpcd_ctx* c) {
-    for (auto& g : c->gexec)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
-}
-
 // the tensor-core kernels' shared memory opt-in and their persistent grid: tiles of 128 rows,
 // at most 4 CTAs per SM
 static int tc_setup(int device, int rows, int* grid) {

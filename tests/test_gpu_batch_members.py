@@ -1,7 +1,8 @@
 """Batches of small replicas that step on their own streams, joined around the zone passes, because a member
 has an option that only its own step implements (mean flow kept, one full-domain zone, the learned closure):
 each replica equals the replica alone, bit for bit, eager and replayed, also when the members' buffers come to
-lie differently."""
+lie differently, when a batch goes over from one kind of step to the other between calls, and when an option
+changes after steps have been captured."""
 import numpy as np
 import pytest
 
@@ -88,5 +89,34 @@ def test_buffers_that_lie_differently_and_alike_again(graphs):
         again = ("state", 50) if i == 1 else ("none",)
         return [("state", 30 + i), ("step", 0, 11), again, ("step", 11, 9), ("read",), ("state", 60 + i),
                 ("step", 20, 10), ("read",)]
+
+    _check(native, _cases("keepMeanFlow"), ops, graphs)
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_learned_closure_switched_between_calls(graphs):
+    """The batch goes over from batched launches to the members' own streams and back."""
+    native = _native()
+
+    def ops(i):
+        def learned(*a):
+            return ("learned", *a) if i == 1 else ("none",)
+        return [("state", 30 + i), ("step", 0, 7), learned(5, 10.0), ("step", 7, 11), ("read",), learned(None),
+                ("step", 18, 6), ("read",), learned(6, 1e-6), ("step", 24, 12), ("read",)]
+
+    _check(native, _cases("learned"), ops, graphs)
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_learned_closure_switched_under_captured_steps(graphs):
+    """A replica with the mean flow kept holds the batch on the members' own streams throughout; the closure
+    of another one changes after the batch's steps have been captured."""
+    native = _native()
+
+    def ops(i):
+        def learned(*a):
+            return ("learned", *a) if i == 2 else ("none",)
+        return [("state", 30 + i), ("step", 0, 12), learned(5, 10.0), ("step", 12, 12), ("read",), learned(6, 1e-6),
+                ("step", 24, 12), ("read",), learned(None), ("step", 36, 10), ("read",)]
 
     _check(native, _cases("keepMeanFlow"), ops, graphs)
