@@ -46,9 +46,7 @@ struct F64Job {
     int n, nwords, nzBase, nzShifted, anyMask, tileCap, nbRed, reserved;
 };
 
-constexpr int kF64CollideShape = 0;     // 32 cells by 128 threads (the tuner's usual choice)
-constexpr int kF64CollideCells = kCollideShape[kF64CollideShape].cells;
-constexpr int kF64CollideThreads = kCollideShape[kF64CollideShape].threads;
+constexpr int kF64CollideShape = 0;     // 32 cells by 128 threads, unless the members agree on another
 constexpr int kF64WallBlocks = 8;       // blocks per replica of the thermal-wall and correction kernels
 
 #define MPCD_F64_JOB(J, blk)                                            \
@@ -129,14 +127,16 @@ __global__ void __launch_bounds__(kSignThreads) k_f64_signs(F64Jobs jobs, long l
         srd_signs_block(0, J.P.Nc, J.signs0, J.stepSeeds, J.signs1);
 }
 
-// dynamic shared memory: the arguments, then the tile
-__global__ void __launch_bounds__(kF64CollideThreads) k_f64_collide(F64Jobs jobs, F64Offs offs, int n) {
+// tile shape K (kCollideShape); dynamic shared memory: the arguments, then the tile
+template <int K>
+__global__ void __launch_bounds__(kCollideShape[K].threads) k_f64_collide(F64Jobs jobs, F64Offs offs, int n) {
     extern __shared__ __align__(16) char smem[];
     const int r = fb_replica(offs, n, (int)blockIdx.x);
     if (r < 0) return;
     const F64Job& J = fb_stage(jobs, r, smem);
-    srd_collide_block<View64, kF64CollideCells>((int)blockIdx.x - offs[r], smem + fb_bytes<F64Job>(), J.P, J.startSrd,
-                                                J.slotsSrd, J.signs0, J.P.Nc, J.S, J.st, J.stepSeeds, J.signs1, J.tileCap);
+    srd_collide_block<View64, kCollideShape[K].cells>((int)blockIdx.x - offs[r], smem + fb_bytes<F64Job>(), J.P, J.startSrd,
+                                                      J.slotsSrd, J.signs0, J.P.Nc, J.S, J.st, J.stepSeeds, J.signs1,
+                                                      J.tileCap);
 }
 
 __global__ void __launch_bounds__(256) k_f64_fields(F64Jobs jobs, F64Offs offs, int n) {
