@@ -103,8 +103,10 @@ struct mpcd_ctx {
     int* pidb[2] = {nullptr, nullptr};
     int xv = 0, pp = 0;
     // Position buffers are addressed as [k ^ xflip] for view index k: the zone passes update
-    // positions in place and velocities out of place, so each pass flips xv and xflip together
-    // (the positions stay in their buffer); a whole step leaves xflip as it found it.
+    // positions in place. A pass with its velocities out of place flips xv and xflip together (the
+    // positions stay in their buffer); the step's shifted pass in place flips neither; the closure's
+    // re-sort flips xv and pp. So a step flips pp and xflip and leaves xv as it found it; with
+    // the shifted pass out of place (shiftInPlace off) it flips pp and xv and leaves xflip.
     int xflip = 0;
     int* redDone = nullptr;   // blocks finished of the reduction in progress (k_reduce_cols resets it)
     int* partFill = nullptr;  // kPartBuckets: bucket fill counts of the state's id-order output (state_io.cuh)
@@ -270,7 +272,9 @@ struct mpcd_ctx {
     int zMaxCells = 0, zWinCap = 0, zArenaCap = 0, zNsmCap = 0;
     int collideShape = -1;     // index into kCollideShape; -1: autotune at the next eager collision
                                // that finds the slots in (cell, id) order
-    bool slotsSorted = false;  // slots in (cell, id) order: false after a state upload until a step
+    // slots in (cell, id) order, up to the shifted pass's few moved particles, which a patched step
+    // leaves in their old cells' runs; false after a state upload until a step
+    bool slotsSorted = false;
     int collideTiles[kCollideShapes] = {};
     size_t zSmem = 0;
     int ovMaxCells = 0, ovWinCap = 0, ovArenaCap = 0, ovNsmCap = 0;

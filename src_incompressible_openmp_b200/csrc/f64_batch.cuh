@@ -3,9 +3,9 @@
 // kernel (the same per-block body, so each replica's state is bit-identical to the replica stepped
 // alone). Each block first copies its replica's arguments into shared memory.
 //
-// A replica's kernels are far too small to fill the GPU, and 40 of them per replica and step made
-// the batch launch-bound: 64 replicas of the ensemble family (15 M particles) took 10.2 ms per step
-// with a stream per replica and a graph of 1,900 launches, 5.3 ms with 44 launches.
+// A replica's kernels are far too small to fill the GPU, and 30 of them per replica and step made
+// the batch launch-bound: 64 replicas of the ensemble family (13.5 M particles) took 10.2 ms per step
+// with a stream per replica and a graph of 1,900 launches; the 36 launches of a step here take 4.8 ms.
 #pragma once
 #include "bc.cuh"
 #include "cells.cuh"
@@ -43,10 +43,13 @@ struct F64Job {
     int* cellOf;
     const int4* rectsBase;
     int *zoneCost, *zoneHist, *zoneOrder;
-    int n, nwords, nzBase, nzShifted, anyMask, tileCap, nbRed, reserved;
+    int n, nwords, nzBase, nzShifted, anyMask, tileCap, nbRed;
 };
 
-constexpr int kF64CollideShape = 0;     // 32 cells by 128 threads, unless the members agree on another
+// The collision's tile shape unless the members share another: 32 cells by 128 threads. ms per step of the
+// ensemble family by shapes 0 to 6: 64 replicas 4.81 4.80 4.91 4.94 4.85 4.84 4.80, 16 replicas 1.76 1.77
+// 1.74 1.72 1.75 1.76 1.76, 4 replicas 0.69 0.71 0.70 0.76 0.72 0.71 0.72.
+constexpr int kF64CollideShape = 0;
 constexpr int kF64WallBlocks = 8;       // blocks per replica of the thermal-wall and correction kernels
 
 #define MPCD_F64_JOB(J, blk)                                            \

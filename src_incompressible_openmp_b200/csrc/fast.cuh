@@ -66,7 +66,6 @@ struct FastParams {
     // n, n < map <=> n < cut, n > map <=> n > flo, floor(map - n) = flo - n for n <= map, and the
     // deficit in units of 2^-12, rint((map - n) 4096), is map12 - 4096 n
     int cut[2][2], flo[2][2];
-    int reserved;
     long long map12[2][2];
     double fqx, fqy;             // body force * dt in grid units (fractional)
     float dtqx, dtqy;            // cell units moved per grid unit of velocity in one step

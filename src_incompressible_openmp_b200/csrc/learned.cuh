@@ -613,7 +613,7 @@ __global__ void k_learned_decide(const double* __restrict__ sums, int Nc, double
 // which takes 16 of the 64 hidden units.
 // Bound by the latency of the phases between the MMAs: a training batch of 512 rows is four
 // tiles on four SMs. With one thread per row and all 64 units, uncoalesced weights and rows a
-// batch took 72 us, now 27.
+// batch took 75 us, now 27.
 //   forward:  Z1 = X W1^T (b1 in operand column 75), a1 = bf16(gelu(Z1));
 //             Z2 = A1 W2^T (b2 in operand column 64 of A1), a2 = gelu(Z2); out = W3 a2 + b3 (FP32)
 //   backward: dout = 2 (out - y / scale) / (batch * 2); dW3, db3 in FP32 on the CUDA cores;

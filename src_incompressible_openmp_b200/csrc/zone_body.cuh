@@ -288,8 +288,8 @@ __device__ __noinline__ int zone_compact(uint8_t* cflags, I* abase, I* head, con
 }
 
 // smoothed occupancy on the zone plus a one-cell ring (src/zone_pass.cpp:296-319):
-// 3x3 binomial weights, renormalised over the in-domain neighbours. Out of line (called at
-// most twice per pass).
+// 3x3 binomial weights, renormalised over the in-domain neighbours. Out of line: called at most twice per
+// pass, and inlined integer sums came out wrong from ptxas 12.9 in the overflow path's 32-bit working set.
 template <typename W, typename I>
 __device__ __noinline__ void zone_compute_nsm(double* nsm, const W* win, const I* cnt, int xs, int ys, int TX,
                                               int TY, int Nx, int Ny, int perx, int pery, int lane) {
@@ -408,15 +408,6 @@ struct ZoneState {
     __device__ __forceinline__ int gx_of(int l) const { return xs + lx_of(l); }
     __device__ __forceinline__ int gy_of(int l) const { return ys + (l - lx_of(l) * TY); }
 
-    __device__ __forceinline__ int cnt_at(int ix, int iy) const {
-        if (in_zone(ix, iy)) return M.len[loc(ix, iy)];
-        int wx = ix - (xs - 2), wy = iy - (ys - 2);
-        if (wx < 0) wx += P().Nx;
-        else if (wx >= TX + 4) wx -= P().Nx;
-        if (wy < 0) wy += P().Ny;
-        else if (wy >= WY) wy -= P().Ny;
-        return M.win[wx * WY + wy];
-    }
     __device__ __forceinline__ int nsm_index(int ix, int iy) const {
         int lx = ix - (xs - 1), ly = iy - (ys - 1);
         if (lx < 0) lx += P().Nx;
@@ -980,7 +971,7 @@ struct ZoneState {
         __syncwarp();
         zone_shuffle_fast(don, nd, rng, lane);
         // One N(0,1) per donor in shuffled order, then scores in parallel (lane k = donor k). The
-        // score 100 align + Nsm + 1e-9 N(0,1) only ranks the donors, and |N(0,1)| stays below 12
+        // score 100 align + Nsm + 1e-9 N(0,1) only ranks the donors, and |N(0,1)| stays below 12.2
         // (r2 >= 2^-106), so the deviates and the last bits of the norm matter only where two
         // scores lie within 3e-8 of each other: the scores come from sqrt(gx^2 + gy^2) (within
         // 1e-12 (1 + |score|) of the reference's) without the deviates, and a ranking with a gap of
