@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <limits>
 #include <map>
 #include <mutex>
@@ -447,6 +448,23 @@ int dalloc(T** p, size_t count) {
     *p = nullptr;
     if (count == 0) count = 1;
     CUDA_TRY(mpcd_device_malloc((void**)p, count * sizeof(T)));
+    return MPCD_OK;
+}
+
+// Several buffers (place, bytes), all or none: after a failure their places are null again, so that the
+// call that made them on first use tries again.
+int dalloc_all(std::initializer_list<std::pair<void**, size_t>> want) {
+    for (auto w = want.begin(); w != want.end(); ++w) {
+        const cudaError_t e = mpcd_device_malloc(w->first, std::max<size_t>(1, w->second));
+        if (e == cudaSuccess) continue;
+        for (auto q = want.begin(); q != w; ++q) {
+            cudaFree(*q->first);
+            *q->first = nullptr;
+        }
+        *w->first = nullptr;
+        cudaGetLastError();
+        return set_err(MPCD_ERR_CUDA, std::string("device memory: ") + cudaGetErrorString(e));
+    }
     return MPCD_OK;
 }
 
@@ -1282,11 +1300,12 @@ static int launch_zone_serial(mpcd_ctx* c, const int4* rects, const int* owner, 
         // some cells, so twice the particles (plus slack) bounds the live-list area
         c->liveCap = 2LL * c->n + 1024;
         if (c->n + c->liveCap >= (1LL << 31)) return set_err(MPCD_ERR_CAPACITY, "serial pass: too many particles");
-        CUDA_TRY(cudaMalloc(&c->slotsLive, sizeof(int) * (size_t)(c->n + c->liveCap)));
-        CUDA_TRY(cudaMalloc(&c->liveCnt, sizeof(int) * (size_t)c->Nc));
-        CUDA_TRY(cudaMalloc(&c->liveStart, sizeof(int) * (size_t)c->Nc));
-        CUDA_TRY(cudaMalloc(&c->liveTop, sizeof(int)));
-        CUDA_TRY(cudaMalloc(&c->duScratch, sizeof(double2) * (size_t)std::max(std::max(c->zMaxCells, c->ovMaxCells), 1)));
+        rc = dalloc_all({{(void**)&c->slotsLive, sizeof(int) * (size_t)(c->n + c->liveCap)},
+                         {(void**)&c->liveCnt, sizeof(int) * (size_t)c->Nc},
+                         {(void**)&c->liveStart, sizeof(int) * (size_t)c->Nc},
+                         {(void**)&c->liveTop, sizeof(int)},
+                         {(void**)&c->duScratch, sizeof(double2) * (size_t)std::max(c->zMaxCells, c->ovMaxCells)}});
+        if (rc) return rc;
     }
     k_zone_seeds<<<(nZones + kSeedZonesPerBlock - 1) / kSeedZonesPerBlock, kSeedZonesPerBlock * 2, 0, c->stream>>>(
         seedBase, nZones, c->seeds, nullptr, kSeedBase); ++c->launches;
@@ -2227,9 +2246,9 @@ int mpcd_zone_kernel_inplace(mpcd_ctx* c, int32_t x0, int32_t x1, int32_t y0, in
     if (rc) return rc;
     CUDA_TRY(cudaSetDevice(c->device));
     if (!c->zkRect) {
-        CUDA_TRY(cudaMalloc(&c->zkRect, sizeof(int4)));
-        CUDA_TRY(cudaMalloc(&c->zkDiag, 8 * sizeof(double)));
-        CUDA_TRY(cudaMalloc(&c->zkOut, 32 * sizeof(double)));
+        rc = dalloc_all({{(void**)&c->zkRect, sizeof(int4)}, {(void**)&c->zkDiag, 8 * sizeof(double)},
+                         {(void**)&c->zkOut, 32 * sizeof(double)}});
+        if (rc) return rc;
     }
     const int4 R = make_int4(x0, x1, y0, y1);
     CUDA_TRY(cudaMemcpyAsync(c->zkRect, &R, sizeof R, cudaMemcpyHostToDevice, c->stream));
@@ -2701,15 +2720,17 @@ static int load_state_async(mpcd_ctx* c, const double2* x, const double2* v) {
 
 static int ensure_job_buffers(mpcd_ctx* c) {
     if (c->up) return MPCD_OK;
-    for (int b = 0; b < 2; ++b) {
-        int rc = dalloc(&c->jobIn[b], 2 * (size_t)c->n);
-        if (!rc) rc = dalloc(&c->jobOut[b], 2 * (size_t)c->n);
+    if (!c->jobIn[0]) {
+        const size_t bytes = 2 * sizeof(double2) * (size_t)c->n;
+        const int rc = dalloc_all({{(void**)&c->jobIn[0], bytes}, {(void**)&c->jobIn[1], bytes},
+                                   {(void**)&c->jobOut[0], bytes}, {(void**)&c->jobOut[1], bytes}});
         if (rc) return rc;
-        for (cudaEvent_t* e : {&c->upDone[b], &c->inFree[b], &c->outReady[b], &c->downDone[b]})
-            CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
-    CUDA_TRY(cudaStreamCreateWithFlags(&c->down, cudaStreamNonBlocking));
-    CUDA_TRY(cudaStreamCreateWithFlags(&c->up, cudaStreamNonBlocking));
+    for (int b = 0; b < 2; ++b)
+        for (cudaEvent_t* e : {&c->upDone[b], &c->inFree[b], &c->outReady[b], &c->downDone[b]})
+            if (!*e) CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    if (!c->down) CUDA_TRY(cudaStreamCreateWithFlags(&c->down, cudaStreamNonBlocking));
+    CUDA_TRY(cudaStreamCreateWithFlags(&c->up, cudaStreamNonBlocking));  // last: it stands for all of them
     return MPCD_OK;
 }
 
@@ -2780,8 +2801,9 @@ int mpcd_profile_reset(mpcd_ctx* c, int32_t enable) {
     CUDA_TRY(cudaSetDevice(c->device));
     const int Ny = c->pc.Ny;
     if (!c->profP) {
-        CUDA_TRY(cudaMalloc(&c->profP, sizeof(unsigned long long) * (size_t)Ny));
-        CUDA_TRY(cudaMalloc(&c->profN, sizeof(unsigned long long) * (size_t)Ny));
+        const size_t bytes = sizeof(unsigned long long) * (size_t)Ny;
+        const int rc = dalloc_all({{(void**)&c->profP, bytes}, {(void**)&c->profN, bytes}});
+        if (rc) return rc;
     }
     CUDA_TRY(cudaMemsetAsync(c->profP, 0, sizeof(unsigned long long) * (size_t)Ny, c->stream));
     CUDA_TRY(cudaMemsetAsync(c->profN, 0, sizeof(unsigned long long) * (size_t)Ny, c->stream));
@@ -3583,11 +3605,11 @@ static int ensure_learned_buffers(mpcd_ctx* c) {
     if (c->lparams) return MPCD_OK;
     int rc = tc_setup(c->device, c->Nc, &c->tcGrid);
     if (rc) return rc;
-    if ((rc = dalloc(&c->lparams, kParams)) || (rc = dalloc(&c->lmode, 1)) || (rc = dalloc(&c->lcount, 2)) ||
-        (rc = dalloc(&c->lsums, 3)) || (rc = dalloc(&c->duLX, (size_t)c->Nc)) || (rc = dalloc(&c->duLY, (size_t)c->Nc)) ||
-        (rc = dalloc(&c->redFeat, (size_t)c->Nc)) || (rc = dalloc(&c->duLSum, 3)))
-        return rc;
-    return MPCD_OK;
+    const size_t Nc = (size_t)c->Nc;
+    return dalloc_all({{(void**)&c->lparams, sizeof(float) * kParams}, {(void**)&c->lmode, sizeof(int)},
+                       {(void**)&c->lcount, 2 * sizeof(long long)}, {(void**)&c->lsums, 3 * sizeof(double)},
+                       {(void**)&c->duLX, sizeof(double) * Nc}, {(void**)&c->duLY, sizeof(double) * Nc},
+                       {(void**)&c->redFeat, sizeof(float4) * Nc}, {(void**)&c->duLSum, 3 * sizeof(unsigned long long)}});
 }
 
 static int step_flags_ok(const mpcd_ctx* c) {
