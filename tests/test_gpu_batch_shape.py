@@ -24,8 +24,10 @@ def _collide_blocks(step):
     with tempfile.NamedTemporaryFile(suffix=".json") as f:
         prof.export_chrome_trace(f.name)
         events = json.load(open(f.name))["traceEvents"]
-    return {(e["args"]["grid"][0], e["args"]["block"][0]) for e in events
-            if e.get("cat") == "kernel" and "k_f64_collide" in e["name"]}
+    kernels = [e for e in events if e.get("cat") == "kernel"]
+    if not kernels:
+        pytest.skip("no kernel trace on this machine")
+    return {(e["args"]["grid"][0], e["args"]["block"][0]) for e in kernels if "k_f64_collide" in e["name"]}
 
 
 def test_batch_uses_its_members_shape():
